@@ -345,7 +345,9 @@ ipb_status run_match(Context* c, const MatchArgs& a) {
   const bool ref = a.precision == IPB_PRECISION_REFERENCE_F32;
   const int path = g_path.load();
   const bool rows = !ref && path == 3 && shift_supported(a);
-  const bool tensor = !ref && !rows && path != 1 && umma_supported(a);
+  // window tiles wherever they apply; the Hankel-row kernel for wider templates
+  const bool window = !ref && path == 0 && window_supported(a);
+  const bool tensor = !ref && !rows && path != 1 && (window || umma_supported(a));
   ipb_status st;
   if (rows) {
     if ((st = ensure(c, c->errw, sizeof(unsigned int), /*zero=*/true)) ||
@@ -357,7 +359,8 @@ ipb_status run_match(Context* c, const MatchArgs& a) {
     const size_t need = ref ? reference_scratch_bytes(a) : exact_cc_scratch_bytes(a);
     if ((st = ensure(c, c->scratch, need))) return st;
   }
-  IPB_CUDA(cudaStreamWaitEvent(a.stream, c->last, 0), "cudaStreamWaitEvent");
+  // a window launch uses no scratch, only the error word (set by atomics)
+  if (!window) IPB_CUDA(cudaStreamWaitEvent(a.stream, c->last, 0), "cudaStreamWaitEvent");
   MatchArgs la = a;
   la.timer = acquire_timer();
   cudaError_t e;
@@ -368,7 +371,8 @@ ipb_status run_match(Context* c, const MatchArgs& a) {
   } else if (tensor) {
     c->tag += 1;
     c->tensor_since_check = true;
-    e = launch_umma(la, static_cast<unsigned int*>(c->errw.p), c->tag);
+    e = window ? launch_window(la, static_cast<unsigned int*>(c->errw.p), c->tag)
+               : launch_umma(la, static_cast<unsigned int*>(c->errw.p), c->tag);
   } else {
     e = ref ? launch_reference(la, c->scratch.p) : launch_exact_cc(la, c->scratch.p);
   }
@@ -378,7 +382,7 @@ ipb_status run_match(Context* c, const MatchArgs& a) {
                (double)a.W * a.H + tp * (a.mask ? 2.0 : 1.0) + 4.0 * Wo * Ho);
   }
   if (e != cudaSuccess) return cuda_fail(e, "template-matching launch");
-  IPB_CUDA(cudaEventRecord(c->last, a.stream), "cudaEventRecord");
+  if (!window) IPB_CUDA(cudaEventRecord(c->last, a.stream), "cudaEventRecord");
   return IPB_OK;
 }
 
@@ -537,8 +541,9 @@ ipb_status host_match_banded(Context* c, const MatchArgs& full, const uint8_t* i
   ipb_status st;
   if ((st = ensure_band_streams(c, nb))) return st;
   const int path = g_path.load();
-  const bool side_by_side =
-      full.precision != IPB_PRECISION_REFERENCE_F32 && path != 1 && path != 3 && umma_supported(full);
+  const bool exact = full.precision != IPB_PRECISION_REFERENCE_F32;
+  const bool window = exact && path == 0 && window_supported(full);
+  const bool side_by_side = window || (exact && path != 1 && path != 3 && umma_supported(full));
   if (side_by_side && (st = ensure(c, c->errw, sizeof(unsigned int), /*zero=*/true))) return st;
   // A copy into page-locked memory returns at once, so a band's score rows are
   // queued as soon as its launch is: they cross while the host still copies
@@ -609,7 +614,8 @@ ipb_status host_match_banded(Context* c, const MatchArgs& full, const uint8_t* i
         a.timer = acquire_timer();
         c->tag += 1;
         c->tensor_since_check = true;
-        const cudaError_t e = launch_umma(a, static_cast<unsigned int*>(c->errw.p), c->tag);
+        const cudaError_t e = window ? launch_window(a, static_cast<unsigned int*>(c->errw.p), c->tag)
+                                     : launch_umma(a, static_cast<unsigned int*>(c->errw.p), c->tag);
         if (a.timer) {
           const double tp = (double)a.w * a.h, Ho_b = a.H - a.h + 1.0;
           note_timed(a.timer, Wo * Ho_b * tp, (double)a.W * a.H + tp * (a.mask ? 2.0 : 1.0) + 4.0 * Wo * Ho_b);

@@ -53,6 +53,14 @@ struct ipb_batch_plan {
     std::vector<ipb::UmmaProblem> probs;
     ipb::UmmaProblem* d_probs = nullptr;
     uint32_t tiles = 0;
+    // groups on the window kernel: their own plan and descriptors instead
+    bool window = false;
+    uint32_t set = 1;
+    ipb::WindowPlan wplan;
+    std::vector<ipb::WindowProblem> wprobs;
+    std::vector<CUtensorMap> wmaps;
+    ipb::WindowProblem* d_wprobs = nullptr;
+    CUtensorMap* d_wmaps = nullptr;
   };
   std::vector<Group> groups;
   // unmasked pairs of one template on the row-operand kernel: up to 8 per
@@ -91,11 +99,15 @@ namespace {
 // Two decisions are tuned and cached per process, and persisted in a text file
 // (IPB_TUNING_FILE, default ~/.cache/imageproc_b200/tuning.txt; an empty
 // IPB_TUNING_FILE keeps them in memory only):
-//  * per batch group (on unless IPB_AUTOTUNE=0): the tensor-memory row width
-//    (the group's natural width or twice it) and the tile height, timed on
-//    the group's own pairs; key = (natural width, masked, tallest template
-//    rounded up to 8, log2 of the group's output positions, log2 of its
-//    largest image side). Line: "group ks0 masked h8 wlog mlog ks nt".
+//  * per batch group (on unless IPB_AUTOTUNE=0): the kernel and its tiles,
+//    timed on the group's own pairs: the Hankel-row kernel's tensor-memory
+//    row width (the group's natural width or twice it), tile height and set
+//    size, or (row width 0) the window kernel's tile rows (plus one: two
+//    image tiles in shared memory) and set size; key = (natural width,
+//    masked, tallest template rounded up to 8, log2 of the group's output
+//    positions, log2 of its largest image side, largest set, plus 100 where
+//    the window kernel was among the candidates).
+//    Line: "group2 ks0 masked h8 wlog mlog set ks nt n".
 //  * per pair shape class (IPB_AUTOTUNE=1): tensor cores or the CUDA-core
 //    kernel, timed on the first pair of each (w, h, masked, normalised).
 //    Line: "pair w h masked norm tensor".
@@ -263,9 +275,71 @@ ipb_status to_status(cudaError_t e, const char* what) {
 // 2 ks0, each tile height) on the group's own pairs and returns the fastest.
 // The timing launches write the pairs' outputs and extremes keys; the
 // caller re-arms the keys afterwards.
+// Descriptors of a window-kernel group: rows = tile rows (+ 1 for two image
+// tiles); false when no plan fits.
+template <class KeysOf>
+bool window_group(const ipb_batch_plan* p, const std::vector<uint32_t>& mem, bool masked, uint32_t rows, uint32_t set,
+                  KeysOf keys_of, ipb_batch_plan::Group& g) {
+  uint32_t wmax = 1, hmax = 1;
+  for (uint32_t i : mem) {
+    if (!window_supported(p->args[i])) return false;
+    wmax = std::max(wmax, p->args[i].w);
+    hmax = std::max(hmax, p->args[i].h);
+  }
+  if (rows < 16 || !window_plan_for(wmax, hmax, masked, rows / 16, 1 + (rows & 1u), g.wplan)) return false;
+  g.window = true;
+  g.set = set;
+  g.wprobs.clear();
+  g.wmaps.assign(mem.size(), CUtensorMap{});
+  for (size_t k = 0; k < mem.size(); ++k)
+    g.wprobs.push_back(window_problem(p->args[mem[k]], g.wplan, keys_of(mem[k]), &g.wmaps[k]));
+  g.tiles = window_make_sets(g.wprobs, g.wmaps, g.wplan, set);
+  return true;
+}
+
+// Device copies of the descriptors when they do not fit the kernel parameters.
+cudaError_t upload_window_group(ipb_batch_plan::Group& g) {
+  if (g.wprobs.size() <= kInlineProblems) return cudaSuccess;
+  cudaError_t e = cudaMalloc(&g.d_wprobs, sizeof(WindowProblem) * g.wprobs.size());
+  if (e == cudaSuccess) e = cudaMalloc(&g.d_wmaps, sizeof(CUtensorMap) * g.wmaps.size());
+  if (e == cudaSuccess)
+    e = cudaMemcpy(g.d_wprobs, g.wprobs.data(), sizeof(WindowProblem) * g.wprobs.size(), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess)
+    e = cudaMemcpy(g.d_wmaps, g.wmaps.data(), sizeof(CUtensorMap) * g.wmaps.size(), cudaMemcpyHostToDevice);
+  return e;
+}
+
+void free_window_group(ipb_batch_plan::Group& g) {
+  if (g.d_wprobs) cudaFree(g.d_wprobs);
+  if (g.d_wmaps) cudaFree(g.d_wmaps);
+  g.d_wprobs = nullptr;
+  g.d_wmaps = nullptr;
+}
+
+cudaError_t launch_window_group(const ipb_batch_plan* p, const ipb_batch_plan::Group& g, unsigned int* sched,
+                                bool stall, cudaStream_t s, KernelTimer* t) {
+  WindowLaunch L{};
+  const uint32_t n = (uint32_t)g.wprobs.size();
+  if (n <= kInlineProblems)
+    for (uint32_t i = 0; i < n; ++i) {
+      L.inl[i] = g.wprobs[i];
+      L.inl_maps[i] = g.wmaps[i];
+    }
+  L.probs = g.d_wprobs;
+  L.maps = g.d_wmaps;
+  L.nprobs = n;
+  L.tiles = g.tiles;
+  L.err = p->d_err;
+  L.tag = p->tag;
+  L.wait_ns = pipeline_wait_ns();
+  L.stall = stall ? 1u : 0u;
+  L.sched = sched;
+  return launch_window_batch(g.wplan, L, s, t);
+}
+
 template <class KeysOf>
 ipb_status tune_group(ipb_batch_plan* p, const std::vector<uint32_t>& mem, uint32_t ks0, bool masked, uint32_t hmax,
-                      uint32_t set, KeysOf keys_of, GroupChoice& best) {
+                      uint32_t set, bool window, KeysOf keys_of, GroupChoice& best) {
   best = GroupChoice{ks0, 0, 1};
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   IPB_TRY(cudaEventCreate(&e0), "event");
@@ -323,6 +397,30 @@ ipb_status tune_group(ipb_batch_plan* p, const std::vector<uint32_t>& mem, uint3
     }
    }
   }
+  if (window) {
+    for (uint32_t sz : sets)
+      for (uint32_t rows : {128u, 129u, 64u, 65u}) {
+        if (masked && (rows & 1u)) continue;  // one image tile only
+        ipb_batch_plan::Group g;
+        if (err != cudaSuccess || !window_group(p, mem, masked, rows, sz, keys_of, g)) continue;
+        err = upload_window_group(g);
+        float ms_best = 1e30f;
+        for (int rep = 0; rep < 3 && err == cudaSuccess; ++rep) {
+          cudaEventRecord(e0, nullptr);
+          err = launch_window_group(p, g, p->d_sched, false, nullptr, nullptr);
+          cudaEventRecord(e1, nullptr);
+          if (err == cudaSuccess) err = cudaEventSynchronize(e1);
+          float ms = 0;
+          if (err == cudaSuccess && rep > 0 && cudaEventElapsedTime(&ms, e0, e1) == cudaSuccess)
+            ms_best = std::min(ms_best, ms);
+        }
+        free_window_group(g);
+        if (err == cudaSuccess && ms_best < best_ms) {
+          best_ms = ms_best;
+          best = GroupChoice{0, rows, sz};
+        }
+      }
+  }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   return to_status(err, "tuning launch");
@@ -331,8 +429,10 @@ ipb_status tune_group(ipb_batch_plan* p, const std::vector<uint32_t>& mem, uint3
 void release(ipb_batch_plan* p) {
   if (p->exec) cudaGraphExecDestroy(p->exec);
   if (p->graph) cudaGraphDestroy(p->graph);
-  for (auto& g : p->groups)
+  for (auto& g : p->groups) {
     if (g.d_probs) cudaFree(g.d_probs);
+    free_window_group(g);
+  }
   for (auto& g : p->rgroups)
     if (g.d_scratch) cudaFree(g.d_scratch);
   for (void* b : {(void*)p->d_keys, (void*)p->d_widths, (void*)p->d_outs, p->d_scratch, p->d_ext_scratch,
@@ -364,20 +464,24 @@ ipb_status enqueue(ipb_batch_plan* p, cudaStream_t s, bool timed, uint32_t* kern
   for (size_t gi = 0; gi < p->groups.size(); ++gi) {
     const ipb_batch_plan::Group& g = p->groups[gi];
     const cudaStream_t gs = side_by_side && gi > 0 ? p->side : s;
-    UmmaLaunch L{};
-    const uint32_t n = (uint32_t)g.probs.size();
-    if (n <= kInlineProblems)
-      for (uint32_t i = 0; i < n; ++i) L.inl[i] = g.probs[i];
-    L.probs = g.d_probs;
-    L.nprobs = n;
-    L.tiles = g.tiles;
-    L.err = p->d_err;
-    L.tag = p->tag;
-    L.wait_ns = pipeline_wait_ns();
-    L.stall = pipeline_stall() ? 1u : 0u;
-    L.sched = p->d_sched + 2 * gi;
     KernelTimer* t = timed && !side_by_side ? acquire_kernel_timer() : nullptr;
-    launch_err = launch_umma_batch(g.plan, L, gs, t);
+    if (g.window) {
+      launch_err = launch_window_group(p, g, p->d_sched + 2 * gi, pipeline_stall(), gs, t);
+    } else {
+      UmmaLaunch L{};
+      const uint32_t n = (uint32_t)g.probs.size();
+      if (n <= kInlineProblems)
+        for (uint32_t i = 0; i < n; ++i) L.inl[i] = g.probs[i];
+      L.probs = g.d_probs;
+      L.nprobs = n;
+      L.tiles = g.tiles;
+      L.err = p->d_err;
+      L.tag = p->tag;
+      L.wait_ns = pipeline_wait_ns();
+      L.stall = pipeline_stall() ? 1u : 0u;
+      L.sched = p->d_sched + 2 * gi;
+      launch_err = launch_umma_batch(g.plan, L, gs, t);
+    }
     if (launch_err != cudaSuccess) break;
     double macs = 0, bytes = 0;
     for (uint32_t i : g.members) {
@@ -545,7 +649,8 @@ ipb_status create(const ipb_pair* pairs, uint32_t n, int precision, bool capture
     cudaMemcpy(p->d_widths, widths.data(), sizeof(uint32_t) * p->nkeys, cudaMemcpyHostToDevice);
     cudaMemcpy(p->d_outs, outs.data(), sizeof(void*) * p->nkeys, cudaMemcpyHostToDevice);
   }
-  if ((e = umma_prepare_kernels()) != cudaSuccess) return fail(to_status(e, "kernel attributes"));
+  if ((e = umma_prepare_kernels()) != cudaSuccess || (e = window_prepare_kernels()) != cudaSuccess)
+    return fail(to_status(e, "kernel attributes"));
   if (!by_key.empty()) {
     // tile counters: two words per launch, reset by each launch's last CTA
     const size_t sched_bytes = sizeof(unsigned int) * 2 * by_key.size();
@@ -578,14 +683,19 @@ ipb_status create(const ipb_pair* pairs, uint32_t n, int precision, bool capture
   // each natural group's (row width, tile height): tuned, or the natural
   // width with the tallest tiles; groups that land on the same (width,
   // height, mask kind) share one launch
-  std::map<std::tuple<bool, uint32_t, uint32_t, uint32_t>, std::vector<uint32_t>> launches;
+  // (window-kernel groups keep their natural width apart: their shared memory
+  // is carved for the launch's largest template)
+  std::map<std::tuple<bool, uint32_t, uint32_t, uint32_t, uint32_t>, std::vector<uint32_t>> launches;
   for (auto& kv : by_key) {
     const std::vector<uint32_t>& mem = kv.second;
     const bool masked = p->args[mem.front()].mask != nullptr;
     const uint32_t ks0 = kv.first / 2;  // umma_group_key = row width * 2 + masked
     const uint32_t set = set_of(mem);
+    bool window = kernel_path() == 0;
+    for (uint32_t i : mem) window = window && window_supported(p->args[i]);
     // untuned: sets of up to four unmasked pairs, two binary-mask pairs
     GroupChoice c{ks0, 0, masked ? std::min(set, 2u) : set};
+    if (window) c = GroupChoice{0, 128, set};
     if (tune) {
       uint32_t hmax = 0, side = 0;
       double pos = 0;
@@ -595,7 +705,8 @@ ipb_status create(const ipb_pair* pairs, uint32_t n, int precision, bool capture
         side = std::max(side, std::max(a.W, a.H));
         pos += (double)(a.W - a.w + 1) * (a.H - a.h + 1);
       }
-      const GroupKey gk{ks0, masked ? 1 : 0, (hmax + 7) & ~7u, floor_log2(pos), floor_log2(side), set};
+      const GroupKey gk{ks0, masked ? 1 : 0, (hmax + 7) & ~7u, floor_log2(pos), floor_log2(side),
+                        set + (window ? 100u : 0u)};
       bool have = false;
       {
         std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -607,14 +718,14 @@ ipb_status create(const ipb_pair* pairs, uint32_t n, int precision, bool capture
         }
       }
       if (!have) {
-        ipb_status st = tune_group(p, mem, ks0, masked, hmax, set, keys_of, c);
+        ipb_status st = tune_group(p, mem, ks0, masked, hmax, set, window, keys_of, c);
         if (st != IPB_OK) return fail(st);
         std::lock_guard<std::mutex> lk(g_tune_mu);
         g_group_tune[gk] = c;
         tune_store_locked();
       }
     }
-    auto& dst = launches[std::make_tuple(masked, c.ks, c.nt, c.set)];
+    auto& dst = launches[std::make_tuple(masked, c.ks, c.nt, c.set, c.ks ? 0u : ks0)];
     dst.insert(dst.end(), mem.begin(), mem.end());
   }
   for (auto& kv : launches) {
@@ -628,6 +739,18 @@ ipb_status create(const ipb_pair* pairs, uint32_t n, int precision, bool capture
     for (uint32_t i : g.members) {
       hmax = std::max(hmax, p->args[i].h);
       ks = std::max(ks, umma_row_width(p->args[i].w));
+    }
+    if (std::get<1>(kv.first) == 0 &&
+        window_group(p, g.members, masked, nt, std::min(std::get<3>(kv.first), set_of(g.members)), keys_of, g)) {
+      g.plan = UmmaPlan{};
+      g.plan.ks = std::get<4>(kv.first);
+      g.plan.masked = masked;
+      if ((e = upload_window_group(g)) != cudaSuccess) {
+        free_window_group(g);
+        return fail(to_status(e, "window descriptors"));
+      }
+      p->groups.push_back(std::move(g));
+      continue;
     }
     // a cached choice that no longer fits falls back to the tallest tiles,
     // then to problems alone
@@ -729,8 +852,8 @@ IPB_API ipb_status ipb_batch_plan_groups(const ipb_batch_plan* plan, uint32_t ma
   const uint32_t n = (uint32_t)plan->groups.size();
   for (uint32_t i = 0; i < n && i < max; ++i) {
     const ipb_batch_plan::Group& g = plan->groups[i];
-    out[i] = ipb_batch_group{g.plan.ks, g.plan.NT, g.plan.masked ? 1 : 0, (uint32_t)g.members.size(), g.tiles,
-                             g.plan.set_max};
+    out[i] = ipb_batch_group{g.plan.ks, g.window ? 16 * g.wplan.nj : g.plan.NT, g.plan.masked ? 1 : 0,
+                             (uint32_t)g.members.size(), g.tiles, g.window ? g.set : g.plan.set_max};
   }
   if (count) *count = n;
   return IPB_OK;

@@ -138,6 +138,39 @@ __device__ __forceinline__ uint32_t norm_bits_fp64_fast(uint32_t s, double w, bo
   return (((hi - (896u << 20)) << 3) | (alo >> 29)) + (dropped >> 28);
 }
 
+// norm_quotient_fp64 without branches, for epilogues that score many values
+// independently: the f32 bits of RN_f32(RN_d(s / RN_d(sqrt(P)))), P = RN_d(Y
+// T), from the same estimate (one Newton-Raphson step on the approximate
+// reciprocal root) with the same bound (fewer than 2^13 units of a's last
+// place) and window (2^16 units). P = fma(2^52 + Y, T, -2^52 T) and a =
+// fma(2^52 + s, r1, -2^52 r1) are the rounded exact products Y T and s r1
+// (integers enter under the exponent of 2^52), and h = r0 / 2 is exact, so
+// five double operations remain. `undecided` is set when the result must
+// come from finish_score32 instead: a inside the window, or Y == 0 (zero
+// norm). s == 0 gives a == 0, whose high word is clamped up so that the bits
+// are those of +0.0f. td = T > 0, tc = -2^52 td.
+__device__ __forceinline__ uint32_t norm_bits_fp64_filter(uint32_t s, uint32_t Y, double td, double tc,
+                                                          bool& undecided) {
+  const double P = __fma_rn(__hiloint2double(0x43300000, (int)Y), td, tc);
+  const uint32_t phi = (uint32_t)__double2hiint(P), plo = (uint32_t)__double2loint(P);
+  const float pf = __uint_as_float(((phi - (896u << 20)) << 3) | (plo >> 29));
+  float rf;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(rf) : "f"(pf));
+  const uint32_t ru = __float_as_uint(rf);
+  const uint32_t rhi = (ru >> 3) + (896u << 20), rlo = ru << 29;
+  const double r0 = __hiloint2double((int)rhi, (int)rlo);
+  const double e = __fma_rn(-__dmul_rn(P, r0), r0, 1.0);
+  const double r1 = __fma_rn(__hiloint2double((int)(rhi - (1u << 20)), (int)rlo), e, r0);
+  const double nc = __hiloint2double((int)((uint32_t)__double2hiint(r1) + 0x83400000u), __double2loint(r1));
+  const double a = __fma_rn(__hiloint2double(0x43300000, (int)s), r1, nc);
+  const uint32_t ahi = (uint32_t)__double2hiint(a), alo = (uint32_t)__double2loint(a);
+  const uint32_t dropped = alo & 0x1FFFFFFFu;
+  undecided |= dropped - (0x10000000u - 0x10000u) < 0x20000u;
+  undecided |= Y == 0u;
+  const uint32_t hi = max(ahi, 896u << 20);
+  return (((hi - (896u << 20)) << 3) | (alo >> 29)) + (dropped >> 28);
+}
+
 // finish_score for callers whose X, Y and TSS are all below 2^31 (templates
 // of at most 33025 pixels): the integer score fits in 32 bits, and SSE's
 // Y + TSS - 2X is exact in wrapping u32 arithmetic because the true result

@@ -6,6 +6,7 @@
 #include <cstdint>
 #include <vector>
 #include <mutex>
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 namespace ipb {
@@ -297,6 +298,66 @@ cudaError_t launch_extremes_keys_init(unsigned long long* keys, uint32_t n, cuda
 // The finish kernel writes the records and re-arms the keys for the next launch.
 cudaError_t launch_extremes_keys_finish(unsigned long long* keys, const uint32_t* widths,
                                         ipb_extremes_f32* const* outs, uint32_t n, cudaStream_t s);
+
+// ---- tensor-core exact kernel with the staged tile as the A operand (tm_window.cu)
+// One problem of a launch (device-side descriptor).
+struct WindowProblem {
+  const uint8_t* img;
+  const uint8_t* tpl;
+  const uint8_t* mask;      // binary mask or null
+  float* out;               // null: extremes only
+  unsigned long long* ext;  // fused find_extremes keys {min, max} or null
+  uint32_t W, H, w, h;
+  uint32_t Wo, Ho, tiles_x, tile_begin;  // tile_begin: first global tile of the problem
+  uint32_t K, pitch;        // bytes per template-block row (w + 15 rounded up to 32), staged image row pitch
+  uint32_t nch, crows;      // chunks of template rows, rows per chunk
+  uint32_t load_mode, tile_bytes;
+  int method, precision;
+  // members of the set this problem leads (0 on the others, which follow it);
+  // whether any member needs the window sums
+  uint32_t set_n, need_y;
+};
+
+struct WindowLaunch {
+  CUtensorMap inl_maps[kInlineProblems];  // images whose rows are 16-byte aligned
+  WindowProblem inl[kInlineProblems];
+  const WindowProblem* probs;  // device arrays when nprobs > kInlineProblems
+  const CUtensorMap* maps;
+  uint32_t nprobs, tiles;
+  uint32_t nj, nbuf, plane_bytes, slot_bytes;
+  uint32_t img_off, b_off, raw_off, raw_bytes;
+  unsigned int* err;
+  unsigned int tag;
+  unsigned long long wait_ns;  // budget of the bounded waits, per tile
+  uint32_t stall;
+  unsigned int* sched;         // as in UmmaLaunch
+};
+
+// Launch-wide plan: 16 nj output rows per tile, image tile buffers, shared-memory carve.
+struct WindowPlan {
+  bool masked;
+  uint32_t nj, nbuf, plane_bytes, slot_bytes, img_off, b_off, raw_off, raw_bytes, smem;
+};
+
+bool window_supported(const MatchArgs& a);
+// Plan for templates up to wmax x hmax; false when it does not fit.
+bool window_plan_for(uint32_t wmax, uint32_t hmax, bool masked, uint32_t nj, uint32_t nbuf, WindowPlan& pl);
+bool window_plan_best(uint32_t wmax, uint32_t hmax, bool masked, uint32_t nj, WindowPlan& pl);
+WindowProblem window_problem(const MatchArgs& a, const WindowPlan& pl, unsigned long long* ext, CUtensorMap* map);
+// Puts each set (up to `most` problems on one image with one template size
+// and mask) in order, numbers the sets' tiles and returns their number.
+uint32_t window_make_sets(std::vector<WindowProblem>& probs, std::vector<CUtensorMap>& maps, const WindowPlan& pl,
+                          uint32_t most);
+uint32_t window_problem_tiles(const WindowProblem& q, const WindowPlan& pl);
+// Sets the kernels' shared-memory limit (outside stream capture).
+cudaError_t window_prepare_kernels();
+// Fills the plan fields of L and launches (inl / probs, nprobs, tiles, err, tag set by the caller).
+cudaError_t launch_window_batch(const WindowPlan& pl, WindowLaunch& L, cudaStream_t stream, KernelTimer* timer);
+cudaError_t launch_window(const MatchArgs& a, unsigned int* err_word, unsigned int tag);
+// n <= kInlineProblems problems of one image, template size and mask in one
+// launch, with find_extremes keys (2 per problem, armed by the caller) or null.
+cudaError_t launch_window_few(const MatchArgs* a, uint32_t n, unsigned long long* keys, unsigned int* err_word,
+                              unsigned int tag, cudaStream_t stream, KernelTimer* timer);
 
 // ---- many templates of one size against one image (tm_many.cu) ------------
 bool many_supported(uint32_t w, uint32_t h, uint32_t n, int precision);

@@ -198,6 +198,20 @@ __device__ __forceinline__ void mma_i8_ss_warp(uint32_t d_tmem, uint64_t a_desc,
       : "memory");
 }
 
+// D[tmem] (+)= A[smem] * B[smem]^T, issued by one thread, descriptors given as
+// their low and high words.
+__device__ __forceinline__ void mma_i8_ss(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo,
+                                          uint32_t b_hi, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
+      "setp.ne.b32 p, %6, 0;\n\t"
+      "mov.b64 a, {%1, %2};\n\t"
+      "mov.b64 b, {%3, %4};\n\t"
+      "tcgen05.mma.cta_group::1.kind::i8 [%0], a, b, %5, p;\n\t}" ::"r"(d_tmem),
+      "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
 // True in exactly one lane of a converged warp.
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred = 0;

@@ -1,0 +1,105 @@
+"""The window kernel (staged image tiles read in place as the A operand)
+against the oracle, bit for bit.
+
+Shapes sit at the kernel's edges: template widths where the K of the MMAs or
+the staged pitch steps (1, 2, 17, 18, 33, 34, 49, 50, 81, 82, 113, 114, 128),
+template heights below, at and above a tile's rows per lane group and at the
+limits of the block slots (1, 7, 8, 9, 64, 65, 127, 128), maps of one row, one
+column, one position, a tile and one more, and image rows on 16-byte, 4-byte
+and odd boundaries.
+"""
+
+import numpy as np
+import pytest
+
+from imageproc_b200 import template_matching as tm
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+M = tm.MatchTemplateMethod
+
+# (image width, height), (template width, height)
+SHAPES = [
+    ((128, 40), (1, 1)), ((255, 33), (2, 7)), ((144, 23), (17, 8)), ((145, 200), (18, 9)),
+    ((161, 97), (33, 65)), ((34, 150), (34, 1)), ((513, 128), (49, 128)), ((178, 177), (50, 50)),
+    ((208, 271), (81, 128)), ((700, 65), (82, 64)), ((1300, 300), (113, 33)), ((113, 1000), (113, 127)),
+    ((242, 143), (114, 16)), ((256, 255), (128, 128)), ((128, 128), (128, 128)), ((1024, 768), (64, 64)),
+    ((2000, 1111), (31, 5)),
+]
+
+
+@pytest.fixture(autouse=True)
+def _restore():
+    old_p, old_path = tm.get_precision(), tm.get_path()
+    tm.set_path(tm.Path.Auto)
+    yield
+    tm.set_precision(old_p)
+    tm.set_path(old_path)
+
+
+def bits(a):
+    return np.ascontiguousarray(a, np.float32).view(np.uint32)
+
+
+def scene(W, H, w, h):
+    g = np.random.default_rng(W * 7 + H * 5 + w * 3 + h)
+    image = g.integers(0, 256, (H, W), dtype=np.uint8)
+    image[: H // 3, : W // 2] = 0  # zero norms
+    image[H // 2:, W // 2:] = 255
+    return image, g.integers(0, 256, (h, w), dtype=np.uint8), (g.random((h, w)) < 0.7).astype(np.uint8)
+
+
+@pytest.mark.parametrize("shape", SHAPES, ids=lambda s: f"{s[0][0]}x{s[0][1]}_t{s[1][0]}x{s[1][1]}")
+def test_window_kernel_bit_exact(shape):
+    (W, H), (w, h) = shape
+    image, template, mask = scene(W, H, w, h)
+    for method in M:
+        for m in (None, mask):
+            got = tm.match_template(image, template, method) if m is None else \
+                tm.match_template_with_mask(image, template, method, m)
+            exp = O.match_exact(image, template, method, m, precision=0)
+            bad = np.argwhere(bits(got) != bits(exp))
+            assert bad.size == 0, (method, m is not None, bad[:3])
+
+
+@pytest.mark.parametrize("offset", [0, 1, 2, 4, 8])
+def test_window_kernel_unaligned_buffers_and_sets(offset, tmp_path, monkeypatch):
+    # images, templates and masks at odd addresses; sets of one image whose
+    # members differ in template, method and need of the window sums, binary
+    # masks among them, untuned so that every group runs on the window kernel
+    import torch
+
+    from imageproc_b200 import _lib, device
+    monkeypatch.setenv("IPB_AUTOTUNE", "0")
+    monkeypatch.setenv("IPB_TUNING_FILE", "")
+    _lib.lib().ipb_batch_tuning_reset()
+
+    def dev(a):
+        buf = torch.zeros(a.size + 64, dtype=torch.uint8, device="cuda")
+        view = buf[offset:offset + a.size].view(a.shape)
+        view.copy_(torch.from_numpy(a))
+        return view
+
+    items, dev_items = [], []
+    for W, H, w, h in ((512, 300, 40, 24), (301, 260, 64, 70), (640, 129, 8, 100)):
+        image, t0, mask = scene(W, H, w, h)
+        t1 = t0[::-1].copy()
+        di, d0, d1, dm = dev(image), dev(t0), dev(t1), dev(mask)
+        for t, d, method in ((t0, d0, 2), (t0, d0, 3), (t1, d1, 0), (t1, d1, 1), (t0, d0, 1)):
+            items += [(image, t, method, None), (image, t, method, mask)]
+            dev_items += [(di, d, method), (di, d, method, dm)]
+    batch = device.Batch(dev_items)
+    plan = device.BatchPlan(batch)
+    for _ in range(2):
+        for o in batch.outs:
+            o.fill_(-1.0)
+        plan.launch()
+        torch.cuda.synchronize()
+        for k, ((image, t, method, mask), out, e) in enumerate(zip(items, batch.outs, batch.extremes_host())):
+            exp = O.match_exact(image, t, method, mask, precision=0)
+            bad = np.argwhere(bits(out.cpu().numpy()) != bits(exp))
+            assert bad.size == 0, (k, bad[:3])
+            mx, mn, mxl, mnl = O.find_extremes(exp)
+            assert (e.max_value, e.min_value, e.max_value_location, e.min_value_location) == \
+                (float(mx), float(mn), mxl, mnl), k
+    plan.close()
