@@ -9,10 +9,25 @@
 // release build; because addition modulo 2^32 is associative, the parallel
 // scans below give the reference's sequential result bit for bit.
 //
-// Two passes over the table: a row scan (one block per row, tiles of 1024
-// pixels scanned block-wide and stored through shared memory in contiguous
-// runs), then a column scan of the (W+1)*C interleaved columns in place (32
-// row segments per block: segment totals, then the rescan with offsets).
+// One channel (sat_strip_sums, sat_strip_cols, sat_tiles): the table is
+// written once. The image is cut into strips of 16 rows and tiles of 1024
+// columns. The first pass reads the image and leaves in each strip's last
+// table row the strip's column sums, prefix-summed along x, and in the tile's
+// own part of each other row the row's sum ahead of the tile. The second
+// sums the strips' last rows down the image (in place: they are final then).
+// The third forms every other row of a tile from the final row above its
+// strip, its rows' sums ahead of the tile and the tile's own two-dimensional
+// prefix (16 rows at once: per-thread runs of four columns, one warp scan and
+// one exchange between warps per row, staged in 32 bits so that warps store
+// contiguous runs). Nothing but the table holds intermediates. The bound is
+// the table's one write: 4096 x 4096 squared u64, 23 us for image and table
+// at the copy rate; two passes over the table 117 us, this 65 us.
+//
+// Three and four channels: two passes over the table: a row scan (one block
+// per row, tiles of 1024 pixels scanned block-wide and stored through shared
+// memory in contiguous runs), then a column scan of the (W+1)*C interleaved
+// columns in place (32 row segments per block: segment totals, then the
+// rescan with offsets).
 #include "tm_common.cuh"
 #include "tm_internal.h"
 
@@ -135,12 +150,256 @@ __global__ void __launch_bounds__(32 * kSegs) sat_cols_kernel(uint32_t cols, uin
   }
 }
 
+constexpr uint32_t kStripRows = 16, kTileCols = 1024, kTileThreads = 256;
+
+// The four pixels of a thread, zero past the image: one word where rows are
+// word-aligned.
+__device__ __forceinline__ uint32_t four_pixels(const uint8_t* __restrict__ row, uint32_t x, uint32_t W, bool aligned) {
+  if (aligned && x + 4 <= W) return __ldg(reinterpret_cast<const uint32_t*>(row + x));
+  uint32_t v = 0;
+#pragma unroll
+  for (uint32_t k = 0; k < 4; ++k)
+    if (x + k < W) v |= (uint32_t)__ldg(row + x + k) << (8 * k);
+  return v;
+}
+template <bool kSquare>
+__device__ __forceinline__ uint32_t term(uint32_t v, int k) {
+  const uint32_t b = (v >> (8 * k)) & 255u;
+  return kSquare ? b * b : b;
+}
+
+// First pass: one block per strip. Sums of up to 16 rows x 1024 columns stay
+// below 2^32 (65025 * 16384).
+template <typename T, bool kSquare>
+__global__ void __launch_bounds__(kTileThreads) sat_strip_sums_kernel(const uint8_t* __restrict__ img, uint32_t W,
+                                                                     uint32_t H, bool aligned, T* __restrict__ sat) {
+  __shared__ uint32_t s_row[kStripRows][kTileThreads / 32];
+  __shared__ uint32_t s_col[kTileThreads / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const size_t pitch = (size_t)W + 1;
+  for (uint32_t strip = blockIdx.x; strip * kStripRows < H; strip += gridDim.x) {
+    const uint32_t y0 = strip * kStripRows, rows = min(kStripRows, H - y0);
+    const bool whole = rows == kStripRows;  // the last row's sums are wanted
+    if (threadIdx.x < rows) sat[(y0 + 1 + threadIdx.x) * pitch] = 0;  // left column
+    T col_carry = 0, row_carry = 0;         // row_carry: thread r's row
+    for (uint32_t tile = 0; tile < W; tile += kTileCols) {
+      const uint32_t x = tile + 4 * threadIdx.x;
+      uint32_t v[kStripRows], c[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+      for (uint32_t r = 0; r < kStripRows; ++r)
+        v[r] = r < rows && x < W ? four_pixels(img + (size_t)(y0 + r) * W, x, W, aligned) : 0u;
+#pragma unroll
+      for (uint32_t r = 0; r < kStripRows; ++r) {
+        uint32_t t;
+        if constexpr (kSquare) t = __dp4a(v[r], v[r], 0u);
+        else t = __dp4a(v[r], 0x01010101u, 0u);
+        t = __reduce_add_sync(0xffffffffu, t);
+        if (lane == 0) s_row[r][warp] = t;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) c[k] += term<kSquare>(v[r], k);
+      }
+      const uint32_t own = c[0] + c[1] + c[2] + c[3];
+      uint32_t incl = own;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t n = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += n;
+      }
+      if (lane == 31) s_col[warp] = incl;
+      __syncthreads();
+      uint32_t off = incl - own, tot = 0;
+#pragma unroll
+      for (int k = 0; k < (int)kTileThreads / 32; ++k) {
+        if (k < warp) off += s_col[k];
+        tot += s_col[k];
+      }
+      if (whole) {
+        T run = col_carry + off;
+        T* dst = sat + (size_t)(y0 + kStripRows) * pitch + 1;
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) {
+          run += c[k];
+          if (x + k < W) dst[x + k] = run;
+        }
+      }
+      col_carry += tot;
+      // rows whose table row is formed by the third pass
+      if (threadIdx.x < (whole ? kStripRows - 1 : rows)) {
+        sat[(size_t)(y0 + 1 + threadIdx.x) * pitch + 1 + tile] = row_carry;
+#pragma unroll
+        for (int k = 0; k < (int)kTileThreads / 32; ++k) row_carry += s_row[threadIdx.x][k];
+      }
+      __syncthreads();  // s_row and s_col are rewritten by the next tile
+    }
+  }
+}
+
+// Second pass: sums the strips' last table rows down the image, 32 columns x
+// 32 segments of strips per block.
+template <typename T>
+__global__ void __launch_bounds__(1024) sat_strip_cols_kernel(uint32_t W, uint32_t strips, T* __restrict__ sat) {
+  __shared__ T s_tot[32][33];
+  const uint32_t col = blockIdx.x * 32 + (threadIdx.x & 31);
+  const int segi = threadIdx.x >> 5;
+  const uint32_t seg = (strips + 31) / 32;
+  const uint32_t s0 = segi * seg, s1 = min(strips, s0 + seg);
+  const size_t step = (size_t)kStripRows * (W + 1);
+  T* p = sat + (size_t)kStripRows * (W + 1) + 1 + col;  // strip 0's last row
+  T tot = 0;
+  if (col < W) {
+#pragma unroll 8
+    for (uint32_t i = s0; i < s1; ++i) tot += p[i * step];
+  }
+  s_tot[segi][threadIdx.x & 31] = tot;
+  __syncthreads();
+  T run = 0;
+  for (int k = 0; k < segi; ++k) run += s_tot[k][threadIdx.x & 31];
+  if (col < W) {
+    uint32_t i = s0;
+    for (; i + 8 <= s1; i += 8) {  // eight rows loaded before any is stored
+      T v[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = p[(i + k) * step];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        run += v[k];
+        p[(i + k) * step] = run;
+      }
+    }
+    for (; i < s1; ++i) {
+      run += p[i * step];
+      p[i * step] = run;
+    }
+  }
+}
+
+// Third pass: one block per tile.
+constexpr uint32_t kTileSmem = kStripRows * kTileCols * 4;
+
+template <typename T, bool kSquare>
+__global__ void __launch_bounds__(kTileThreads) sat_tiles_kernel(const uint8_t* __restrict__ img, uint32_t W,
+                                                                uint32_t H, uint32_t tiles_x, bool aligned,
+                                                                T* __restrict__ sat) {
+  extern __shared__ __align__(16) uint32_t s_tile[];  // [kStripRows][kTileCols] prefix within the tile
+  __shared__ uint32_t s_warp[kStripRows][kTileThreads / 32];
+  __shared__ T s_ahead[kStripRows];  // sum of the strip's rows so far, ahead of the tile
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const size_t pitch = (size_t)W + 1;
+  const uint32_t strip = blockIdx.x / tiles_x, tile = (blockIdx.x - strip * tiles_x) * kTileCols;
+  const uint32_t y0 = strip * kStripRows, rows = min(kStripRows, H - y0);
+  const uint32_t form = rows == kStripRows ? kStripRows - 1 : rows;  // the whole strip's last row is final
+  const uint32_t x = tile + 4 * threadIdx.x;
+  uint32_t v[kStripRows];
+#pragma unroll
+  for (uint32_t r = 0; r < kStripRows; ++r)
+    v[r] = r < form && x < W ? four_pixels(img + (size_t)(y0 + r) * W, x, W, aligned) : 0u;
+  // the row above the strip, in the columns this thread stores
+  T base[4];
+#pragma unroll
+  for (uint32_t k = 0; k < 4; ++k) {
+    const uint32_t c = tile + threadIdx.x + k * kTileThreads;
+    base[k] = strip && c < W ? sat[(size_t)y0 * pitch + 1 + c] : T(0);
+  }
+  if (warp == 0) {
+    T ahead = lane < (int)form ? sat[(size_t)(y0 + 1 + lane) * pitch + 1 + tile] : T(0);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const T n = __shfl_up_sync(0xffffffffu, ahead, o);
+      if (lane >= o) ahead += n;
+    }
+    if (lane < (int)kStripRows) s_ahead[lane] = ahead;
+  }
+  uint32_t c0 = 0, c1 = 0, c2 = 0, c3 = 0, own[kStripRows], excl[kStripRows];
+#pragma unroll
+  for (uint32_t r = 0; r < kStripRows; ++r) {
+    c0 += term<kSquare>(v[r], 0);
+    c1 += term<kSquare>(v[r], 1);
+    c2 += term<kSquare>(v[r], 2);
+    c3 += term<kSquare>(v[r], 3);
+    own[r] = c0 + c1 + c2 + c3;
+    excl[r] = own[r];
+  }
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+#pragma unroll
+    for (uint32_t r = 0; r < kStripRows; ++r) {
+      const uint32_t n = __shfl_up_sync(0xffffffffu, excl[r], o);
+      if (lane >= o) excl[r] += n;
+    }
+  }
+#pragma unroll
+  for (uint32_t r = 0; r < kStripRows; ++r) {
+    if (lane == 31) s_warp[r][warp] = excl[r];
+    excl[r] -= own[r];
+  }
+  __syncthreads();  // also: every read of the table above is done before any store below
+  c0 = c1 = c2 = c3 = 0;
+#pragma unroll
+  for (uint32_t r = 0; r < kStripRows; ++r) {
+    uint32_t run = excl[r];
+#pragma unroll
+    for (int k = 0; k < (int)kTileThreads / 32; ++k)
+      if (k < warp) run += s_warp[r][k];
+    c0 += term<kSquare>(v[r], 0);
+    c1 += term<kSquare>(v[r], 1);
+    c2 += term<kSquare>(v[r], 2);
+    c3 += term<kSquare>(v[r], 3);
+    uint4 q;
+    q.x = run + c0;
+    q.y = q.x + c1;
+    q.z = q.y + c2;
+    q.w = q.z + c3;
+    *reinterpret_cast<uint4*>(s_tile + r * kTileCols + 4 * threadIdx.x) = q;
+  }
+  __syncthreads();
+#pragma unroll 4
+  for (uint32_t r = 0; r < form; ++r) {
+    const T ahead = s_ahead[r];
+    T* dst = sat + (size_t)(y0 + 1 + r) * pitch + 1 + tile;
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) {
+      const uint32_t c = threadIdx.x + k * kTileThreads;
+      if (tile + c < W) dst[c] = base[k] + ahead + (T)s_tile[r * kTileCols + c];
+    }
+  }
+}
+
+template <typename T, bool kSquare>
+cudaError_t launch_sat_one_channel(const uint8_t* img, uint32_t W, uint32_t H, T* sat, cudaStream_t s) {
+  const uint32_t strips = (H + kStripRows - 1) / kStripRows, whole = H / kStripRows;
+  const uint32_t tiles_x = (W + kTileCols - 1) / kTileCols;
+  const bool aligned = W % 4 == 0 && (reinterpret_cast<uintptr_t>(img) & 3u) == 0;
+  static PerDeviceOnce attr;
+  cudaError_t e = attr.run([] {
+    return cudaFuncSetAttribute(sat_tiles_kernel<T, kSquare>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)kTileSmem);
+  });
+  if (e != cudaSuccess) return e;
+  sat_strip_sums_kernel<T, kSquare><<<strips < 65535u ? strips : 65535u, kTileThreads, 0, s>>>(img, W, H, aligned,
+                                                                                             sat);
+  count_launch(kKernelIntegralRows);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  if (whole > 1) {
+    sat_strip_cols_kernel<T><<<(W + 31) / 32, 1024, 0, s>>>(W, whole, sat);
+    count_launch(kKernelIntegralCols);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  }
+  sat_tiles_kernel<T, kSquare><<<strips * tiles_x, kTileThreads, kTileSmem, s>>>(img, W, H, tiles_x, aligned, sat);
+  count_launch(kKernelIntegralCols);
+  return cudaGetLastError();
+}
+
 template <typename T, bool kSquare, int C>
 cudaError_t launch_sat_typed(const uint8_t* img, uint32_t W, uint32_t H, T* sat, cudaStream_t s) {
   const uint32_t cols = (W + 1) * C;
   cudaError_t e = cudaMemsetAsync(sat, 0, sizeof(T) * cols, s);  // top row
   if (e != cudaSuccess || H == 0) return e;
   if (W == 0) return cudaMemsetAsync(sat, 0, sizeof(T) * (size_t)cols * (H + 1), s);
+  if constexpr (C == 1) {
+    // tiles are counted in 31 bits
+    if ((uint64_t)((H + kStripRows - 1) / kStripRows) * ((W + kTileCols - 1) / kTileCols) < 0x7FFFFFFFull)
+      return launch_sat_one_channel<T, kSquare>(img, W, H, sat, s);
+  }
   sat_rows_kernel<T, kSquare, C><<<H < 65535u ? H : 65535u, kRowThreads, 0, s>>>(img, W, H, sat);
   count_launch(kKernelIntegralRows);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
