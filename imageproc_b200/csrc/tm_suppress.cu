@@ -203,132 +203,133 @@ __global__ void __launch_bounds__(256) snm_cols_tile_kernel(const T* __restrict_
   }
 }
 
-// One-pass form for element types of 4 bytes or less and radii up to 16: a
-// block owns 128 output columns x 32 output rows, stages the keys of that
-// tile and its r halo once, and runs both window passes in shared memory.
-// Each element's rank is one 64-bit word, (key << 32) | (0xFFFF - col) << 16 |
-// (0xFFFF - row) in tile-local coordinates, so the plain maximum is the
-// reference's winner (largest value, then smaller x, then smaller y) and 0
-// stands for the clipped-away cells outside the image. Both passes find
-// window maxima by van Herk / Gil-Werman: a thread owns k = 2r + 1
-// consecutive outputs, keeps the suffix maxima of their first inputs in
-// registers and sweeps the prefix maxima of the next k, so each output
-// costs two maxima whatever the radius (instead of a scan of 2r + 1).
-constexpr uint32_t kFusedTW = 128, kFusedTH = 32, kFusedThreads = 256;
+// One-pass form for element types of 4 bytes or less and radii 1 to 16: a
+// block owns 128 output columns x 32 output rows. Everything is compiled for
+// the radius. With U and D the maxima of the r cells above and below a pixel,
+// its column window's maximum is C = max(U, own, D); with L and E the maxima
+// of the r values C to its left and right, the pixel is its window's winner
+// (largest value, then smaller x, then smaller y) exactly when own > U, own >=
+// D, own > L and own >= E: equal values to the left or above precede it.
+// Column pass: a thread owns one column of the tile and its r halo, has all
+// 32 + 2r loads in flight at once and forms the maxima of its runs of r cells
+// in registers by van Herk / Gil-Werman (suffix maxima of one run, prefix
+// maxima of the next: three maxima per run whatever the radius). Row pass: a
+// thread owns 32 outputs of one row, the same way, and notes the winners in a
+// bit mask. Values compare as 32-bit keys, 0 standing for the cells outside
+// the image: a pixel of key 0 loses to them and to its equals, which is right
+// for all but the image's first pixel (see the row pass).
+// 4065 x 4065 f32, r = 8 (20 us at the copy rate): with ranks of 64 bits (key,
+// x, y) and a radius of the call, both passes in shared memory, 152 us; this
+// 65 us, 28 instructions per pixel at 42 % occupancy (shared memory).
+constexpr int kFusedTW = 128, kFusedTH = 32, kFusedThreads = 160;
 
-template <uint32_t KMAX, typename In, typename Emit>
-__device__ __forceinline__ void vhgw_run(uint32_t k, uint32_t n_in, uint32_t n_out, const uint32_t base,
-                                         uint64_t (&h)[KMAX], const In& in, const Emit& emit) {
-  // suffix maxima of inputs base .. base + k - 1
-  uint64_t run = 0;
+// m[i] = max of a[i .. i + R - 1]
+template <int R, int NIN, int NOUT>
+__device__ __forceinline__ void run_maxima(const uint32_t (&a)[NIN], uint32_t (&m)[NOUT]) {
+  static_assert(NOUT + R - 1 <= NIN, "runs inside the input");
 #pragma unroll
-  for (int t = KMAX - 1; t >= 0; --t)
-    if ((uint32_t)t < k) {
-      const uint32_t c = base + t;
-      const uint64_t v = c < n_in ? in(c) : 0ull;
-      run = v > run ? v : run;
-      h[t] = run;
-    }
-  // prefix maxima of inputs base + k .. base + 2k - 2, merged into the outputs
-  run = 0;
+  for (int base = 0; base < NOUT; base += R) {
+    uint32_t run = 0;
 #pragma unroll
-  for (uint32_t t = 0; t < KMAX; ++t)
-    if (t < k) {
-      const uint32_t o = base + t;
-      if (o < n_out) emit(o, h[t] > run ? h[t] : run);
-      const uint32_t c = base + k + t;
-      const uint64_t v = c < n_in ? in(c) : 0ull;
-      run = v > run ? v : run;
+    for (int t = R - 1; t >= 0; --t) {
+      if (base + t < NIN) run = max(run, a[base + t]);
+      if (base + t < NOUT) m[base + t] = run;
     }
-}
-
-template <typename T>
-__device__ __forceinline__ T from_okey(uint32_t k) {
-  if constexpr (std::is_same<T, float>::value) {
-    return __uint_as_float((k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k);
-  } else if constexpr (std::is_signed<T>::value) {
-    return (T)(int32_t)(k ^ 0x80000000u);
-  } else {
-    return (T)k;
+    run = 0;
+#pragma unroll
+    for (int t = 1; t < R; ++t) {
+      if (base + R + t - 1 < NIN) run = max(run, a[base + R + t - 1]);
+      if (base + t < NOUT) m[base + t] = max(m[base + t], run);
+    }
   }
 }
 
-template <typename T, uint32_t KMAX>
-__global__ void __launch_bounds__(kFusedThreads) snm_fused_kernel(const T* __restrict__ img, uint32_t W, uint32_t H,
-                                                                  uint32_t r, T* __restrict__ out) {
-  static_assert(sizeof(T) <= 4, "32-bit keys");
-  extern __shared__ __align__(16) unsigned char s_raw[];
-  const uint32_t k = 2 * r + 1;
-  const uint32_t ic = kFusedTW + 2 * r, ir = kFusedTH + 2 * r;
-  uint64_t* s_row = reinterpret_cast<uint64_t*>(s_raw);            // [ir][kFusedTW] row-window winners
-  uint32_t* s_key = reinterpret_cast<uint32_t*>(s_row + ir * kFusedTW);  // [ir][ic] keys
+// Order-preserving key of an element's bits: `flip` is the sign bit of a
+// signed type, `fmask` all ones for f32 (negative values have every bit
+// flipped).
+struct KeyMap {
+  uint32_t flip, fmask;
+  __device__ __forceinline__ uint32_t key(uint32_t raw) const {
+    return raw ^ (flip | ((uint32_t)((int32_t)raw >> 31) & fmask));
+  }
+  __device__ __forceinline__ uint32_t raw(uint32_t key) const {
+    return key ^ (flip | (~(uint32_t)((int32_t)key >> 31) & fmask));
+  }
+};
+
+template <typename U, int R>
+__global__ void __launch_bounds__(kFusedThreads) snm_fused_kernel(const U* __restrict__ img, uint32_t W, uint32_t H,
+                                                                  KeyMap km, U* __restrict__ out) {
+  constexpr int IC = kFusedTW + 2 * R, IR = kFusedTH + 2 * R;
+  constexpr int kColPitch = IC + 1, kKeyPitch = kFusedTW + 1;  // odd: lanes that own rows reach every bank
+  __shared__ uint32_t s_col[kFusedTH * kColPitch];             // column-window maxima C
+  __shared__ uint32_t s_key[kFusedTH * kKeyPitch];             // keys of the winners of their columns, else 0
+  __shared__ uint32_t s_win[kFusedTH][4];                      // winners
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const long long x0 = (long long)blockIdx.x * kFusedTW, y0 = (long long)blockIdx.y * kFusedTH;
-  const long long gx0 = x0 - r, gy0 = y0 - r;
-  // stage the keys; cells outside the image are never read as keys (their
-  // rank is 0, decided from the coordinates)
-  for (uint32_t idx = threadIdx.x; idx < ir * ic; idx += kFusedThreads) {
-    const uint32_t i = idx / ic, c = idx - i * ic;
-    const long long gy = gy0 + i, gx = gx0 + c;
-    uint32_t key = 0;
-    if (gy >= 0 && gy < (long long)H && gx >= 0 && gx < (long long)W) key = okey(img[(size_t)gy * W + gx]);
-    s_key[idx] = key;
+  if (tid < IC) {
+    const long long gx = x0 - R + tid;
+    const bool in = gx >= 0 && gx < (long long)W;
+    const U* p = img + (in ? gx : 0) + (y0 - R) * (long long)W;
+    uint32_t a[IR], u[kFusedTH + R + 1];
+#pragma unroll
+    for (int i = 0; i < IR; ++i) {
+      const long long gy = y0 - R + i;
+      a[i] = in && gy >= 0 && gy < (long long)H ? km.key(p[(size_t)i * W]) : 0u;
+    }
+    run_maxima<R>(a, u);
+    const bool centre = tid >= R && tid < R + kFusedTW;
+#pragma unroll
+    for (int j = 0; j < kFusedTH; ++j) {
+      const uint32_t own = a[j + R], up = u[j], down = u[j + R + 1];
+      s_col[j * kColPitch + tid] = max(own, max(up, down));
+      if (centre) s_key[j * kKeyPitch + tid - R] = own > up && own >= down ? own : 0u;
+    }
   }
   __syncthreads();
-  // row pass: for tile-local row i and output column o, the winner of input
-  // columns o .. o + 2r
-  const uint32_t nseg = (kFusedTW + k - 1) / k;
-  const long long col_lo = -gx0, col_hi = (long long)W - gx0;  // local columns inside the image
-  for (uint32_t task = threadIdx.x; task < ir * nseg; task += kFusedThreads) {
-    const uint32_t i = task / nseg, seg = task - i * nseg;
-    const long long gy = gy0 + i;
-    const bool row_in = gy >= 0 && gy < (long long)H;
-    const uint32_t* kr = s_key + i * ic;
-    const uint64_t rowbits = 0xFFFFu - i;
-    uint64_t h[KMAX];
-    vhgw_run<KMAX>(
-        k, ic, kFusedTW, seg * k, h,
-        [&](uint32_t c) -> uint64_t {
-          if (!row_in || (long long)c < col_lo || (long long)c >= col_hi) return 0ull;
-          return ((uint64_t)kr[c] << 32) | ((uint64_t)(0xFFFFu - c) << 16) | rowbits;
-        },
-        [&](uint32_t o, uint64_t v) { s_row[i * kFusedTW + o] = v; });
+  if (warp < 4) {
+    uint32_t a[IR], m[kFusedTH + R + 1];
+    const uint32_t* row = s_col + lane * kColPitch + 32 * warp;
+#pragma unroll
+    for (int i = 0; i < IR; ++i) a[i] = row[i];
+    run_maxima<R>(a, m);
+    const uint32_t* own = s_key + lane * kKeyPitch + 32 * warp;
+    uint32_t bits = 0;
+#pragma unroll
+    for (int t = 0; t < 32; ++t) {
+      const uint32_t k = own[t];
+      bits |= k > m[t] && k >= m[t + R + 1] ? 1u << t : 0u;
+    }
+    // the image's first pixel wins a window of lowest values: nothing precedes it
+    if (x0 == 0 && y0 == 0 && tid == 0 && a[R] == 0u && m[R + 1] == 0u) bits |= 1u;
+    s_win[lane][warp] = bits;
   }
   __syncthreads();
-  // column pass: for output (o, j), the winner of row winners j .. j + 2r of
-  // column o; the pixel keeps its value iff it is that winner
-  const uint32_t nseg2 = (kFusedTH + k - 1) / k;
-  for (uint32_t task = threadIdx.x; task < kFusedTW * nseg2; task += kFusedThreads) {
-    const uint32_t o = task % kFusedTW, seg = task / kFusedTW;
-    const long long gx = x0 + o;
-    if (gx >= (long long)W) continue;
-    uint64_t h[KMAX];
-    vhgw_run<KMAX>(
-        k, ir, kFusedTH, seg * k, h, [&](uint32_t i) -> uint64_t { return s_row[i * kFusedTW + o]; },
-        [&](uint32_t j, uint64_t v) {
-          const long long gy = y0 + j;
-          if (gy >= (long long)H) return;
-          const uint32_t own = ((0xFFFFu - (o + r)) << 16) | (0xFFFFu - (j + r));
-          out[(size_t)gy * W + gx] = (uint32_t)v == own ? from_okey<T>((uint32_t)(v >> 32)) : T(0);
-        });
+  for (int j = warp; j < kFusedTH; j += kFusedThreads / 32) {
+    const long long gy = y0 + j;
+    if (gy >= (long long)H) break;
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      const int o = 32 * g + lane;
+      if (x0 + o < (long long)W)
+        out[(size_t)gy * W + x0 + o] = (s_win[j][g] >> lane) & 1u ? (U)km.raw(s_key[j * kKeyPitch + o]) : U(0);
+    }
   }
 }
 
-size_t snm_fused_smem(uint32_t r) {
-  return (size_t)(kFusedTH + 2 * r) * (kFusedTW * 8 + (kFusedTW + 2 * r) * 4);
-}
-
-template <typename T, uint32_t KMAX>
-cudaError_t launch_snm_fused(const T* img, uint32_t W, uint32_t H, uint32_t r, T* out, cudaStream_t s) {
-  static PerDeviceOnce attr;
-  cudaError_t e = attr.run([] {
-    return cudaFuncSetAttribute(snm_fused_kernel<T, KMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)snm_fused_smem((KMAX - 1) / 2));
-  });
-  if (e != cudaSuccess) return e;
+template <typename U, int R>
+cudaError_t launch_snm_fused(const U* img, uint32_t W, uint32_t H, KeyMap km, U* out, cudaStream_t s) {
   const dim3 grid((W + kFusedTW - 1) / kFusedTW, (H + kFusedTH - 1) / kFusedTH);
-  snm_fused_kernel<T, KMAX><<<grid, kFusedThreads, snm_fused_smem(r), s>>>(img, W, H, r, out);
+  snm_fused_kernel<U, R><<<grid, kFusedThreads, 0, s>>>(img, W, H, km, out);
   count_launch(kKernelSuppress);
   return cudaGetLastError();
+}
+
+template <typename U, int R = 16>
+cudaError_t launch_snm_radius(const U* img, uint32_t W, uint32_t H, uint32_t r, KeyMap km, U* out, cudaStream_t s) {
+  if (r == (uint32_t)R) return launch_snm_fused<U, R>(img, W, H, km, out, s);
+  if constexpr (R > 1) return launch_snm_radius<U, R - 1>(img, W, H, r, km, out, s);
+  else return cudaErrorInvalidValue;
 }
 
 template <typename T>
@@ -339,10 +340,12 @@ cudaError_t launch_snm_t(const T* img, uint32_t W, uint32_t H, uint32_t r, T* ou
   // apart from the image; tiles are counted in 16 bits (rows of grid.y)
   if constexpr (sizeof(T) <= 4) {
     const bool apart = (const void*)img != (const void*)out;
-    if (apart && r <= 16 && (H + kFusedTH - 1) / kFusedTH <= 65535u) {
-      if (r <= 4) return launch_snm_fused<T, 9>(img, W, H, r, out, s);
-      if (r <= 8) return launch_snm_fused<T, 17>(img, W, H, r, out, s);
-      return launch_snm_fused<T, 33>(img, W, H, r, out, s);
+    if (apart && r >= 1 && r <= 16 && (H + kFusedTH - 1) / kFusedTH <= 65535u) {
+      using U = typename std::conditional<sizeof(T) == 1, uint8_t,
+                                          typename std::conditional<sizeof(T) == 2, uint16_t, uint32_t>::type>::type;
+      const bool real = std::is_same<T, float>::value;
+      const KeyMap km{std::is_signed<T>::value ? 1u << (8 * sizeof(T) - 1) : 0u, real ? 0xFFFFFFFFu : 0u};
+      return launch_snm_radius<U>(reinterpret_cast<const U*>(img), W, H, r, km, reinterpret_cast<U*>(out), s);
     }
   }
   uint32_t* bx = static_cast<uint32_t*>(scratch);
