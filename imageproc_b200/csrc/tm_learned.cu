@@ -6,6 +6,7 @@
 // and loaded with ldmatrix); layer 1 (one input channel, 9 taps), the
 // embedding head of training, the softmax loss and Adam run on CUDA cores.
 // Backward passes treat the bf16 roundings of the forward pass as the identity.
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -291,50 +292,29 @@ __global__ void __launch_bounds__(256) conv_mma_kernel(const uint4* __restrict__
 
 // ---- weight gradients on tensor cores ----------------------------------------------
 // dW[co][ci][ky][kx] += sum_p dZ[p][co] A[p + (ky-1, kx-1)][ci], db[co] += sum_p dZ[p][co]
-// over a tile of 4 rows x 64 pixels: M = output channels (two m-tiles), N =
-// input channels (four n-tiles), K = 16 pixels per step. The 18 (tap, m-tile)
-// pairs are shared out over the 8 warps.
+// over tiles of 256 pixels (4 rows x 64, 8 x 32 or 16 x 16, by the image's
+// width): M = output channels (two m-tiles), N = input channels (four
+// n-tiles), K = 16 pixels per step. The 18 (tap, m-tile) pairs are shared out
+// over the 8 warps. A block goes through many tiles and adds its 9216 sums
+// once, staged in the gradient's order so that warps add contiguous 16-byte
+// runs. A block per tile with one scattered atomic per sum spent its time on
+// those: a layer of 128 crops of 24 x 24 135 us, now 22 us.
+constexpr int kGPix = 256;
+constexpr int kGIn = 18 * 18 > 10 * 34 ? (18 * 18 > 6 * 66 ? 18 * 18 : 6 * 66) : (10 * 34 > 6 * 66 ? 10 * 34 : 6 * 66);
 struct GradSmem {
-  uint4 dz[kTH][kChunks][kTW];         // 16384 B
-  uint4 a[kTH + 2][kChunks][kInW];     // 25344 B
+  uint4 dz[kChunks][kGPix];   // 16384 B
+  uint4 a[kChunks][kGIn];     // 25344 B; both are reused to stage the sums
 };
+static_assert(sizeof(GradSmem) >= 9 * kC * kC * 4, "staged sums");
 
+// 2^lcols columns, 2^(8 - lcols) rows per tile
 __global__ void __launch_bounds__(256) conv_grad_kernel(const uint4* __restrict__ dz, const uint4* __restrict__ act,
-                                                        uint32_t H, uint32_t W, float* __restrict__ dW,
+                                                        uint32_t H, uint32_t W, uint32_t lcols, uint32_t tiles_x,
+                                                        uint32_t tiles_y, uint32_t tiles, float* __restrict__ dW,
                                                         float* __restrict__ db) {
   __shared__ __align__(16) GradSmem sm;
-  const uint32_t n = blockIdx.z;
-  const int y0 = blockIdx.y * kTH, x0 = blockIdx.x * kTW;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  for (int i = tid; i < kTH * kChunks * kTW; i += 256) {
-    const int px = i % kTW, c = (i / kTW) % kChunks, r = i / (kTW * kChunks);
-    const int y = y0 + r, x = x0 + px;
-    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (y < (int)H && x < (int)W) v = dz[(((size_t)n * H + y) * kChunks + c) * W + x];
-    sm.dz[r][c][px] = v;
-  }
-  for (int i = tid; i < (kTH + 2) * kChunks * kInW; i += 256) {
-    const int px = i % kInW, c = (i / kInW) % kChunks, r = i / (kInW * kChunks);
-    const int y = y0 - 1 + r, x = x0 - 1 + px;
-    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (y >= 0 && y < (int)H && x >= 0 && x < (int)W) v = act[(((size_t)n * H + y) * kChunks + c) * W + x];
-    sm.a[r][c][px] = v;
-  }
-  __syncthreads();
-
-  // bias gradient: thread (co, part) sums 32 of the tile's 256 pixels
-  {
-    const int co = tid & 31, part = tid >> 5;
-    float s = 0.f;
-    for (int p = part * 32; p < part * 32 + 32; ++p) {
-      const uint4 u = sm.dz[p / kTW][co >> 3][p % kTW];
-      const uint32_t wd[4] = {u.x, u.y, u.z, u.w};
-      const uint32_t word = wd[(co & 7) >> 1];
-      s += bf2f((uint16_t)((co & 1) ? (word >> 16) : (word & 0xFFFF)));
-    }
-    if (s != 0.f) atomicAdd(db + co, s);
-  }
-
+  const int cols = 1 << lcols, rows = kGPix >> lcols, inw = cols + 2;
   constexpr int kMaxPairs = 3;
   int npairs = 0;
   int ptap[kMaxPairs], pm[kMaxPairs];
@@ -345,7 +325,7 @@ __global__ void __launch_bounds__(256) conv_grad_kernel(const uint4* __restrict_
     pm[k] = q & 1;
     if (q < 18) npairs = k + 1;
   }
-  float acc[kMaxPairs][4][4];
+  float acc[kMaxPairs][4][4], bias = 0.f;
 #pragma unroll
   for (int k = 0; k < kMaxPairs; ++k)
 #pragma unroll
@@ -353,47 +333,89 @@ __global__ void __launch_bounds__(256) conv_grad_kernel(const uint4* __restrict_
 #pragma unroll
       for (int e = 0; e < 4; ++e) acc[k][j][e] = 0.f;
 
-  const int lrow = lane & 7, lm = lane >> 3;
-#pragma unroll 1
-  for (int r = 0; r < kTH; ++r) {
-#pragma unroll 1
-    for (int xs = 0; xs < kTW; xs += 16) {
+  for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const uint32_t n = tile / (tiles_x * tiles_y), rem = tile - n * tiles_x * tiles_y;
+    const int y0 = (int)(rem / tiles_x) * rows, x0 = (int)(rem % tiles_x) * cols;
+    __syncthreads();
+    // a warp stages whole (row, chunk) runs
+#pragma unroll 4
+    for (int i = tid; i < kChunks * kGPix; i += 256) {
+      const int c = i >> 8, p = i & 255, y = y0 + (p >> lcols), x = x0 + (p & (cols - 1));
+      uint4 v = make_uint4(0u, 0u, 0u, 0u);
+      if (y < (int)H && x < (int)W) v = dz[(((size_t)n * H + y) * kChunks + c) * W + x];
+      sm.dz[c][p] = v;
+    }
+    for (int rc = warp; rc < (rows + 2) * kChunks; rc += 8) {
+      const int r = rc >> 2, c = rc & 3, y = y0 - 1 + r;
+      const uint4* src = act + (((size_t)n * H + (y >= 0 && y < (int)H ? y : 0)) * kChunks + c) * W;
+#pragma unroll 3
+      for (int px = lane; px < inw; px += 32) {
+        const int x = x0 - 1 + px;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (y >= 0 && y < (int)H && x >= 0 && x < (int)W) v = src[x];
+        sm.a[c][r * inw + px] = v;
+      }
+    }
+    __syncthreads();
+
+    // bias gradient: thread (co, part) sums an eighth of the tile's pixels
+    {
+      const int co = tid & 31, part = tid >> 5;
+#pragma unroll 4
+      for (int p = part * 32; p < part * 32 + 32; ++p) {
+        const uint4 u = sm.dz[co >> 3][p];
+        const uint32_t wd[4] = {u.x, u.y, u.z, u.w};
+        const uint32_t word = wd[(co & 7) >> 1];
+        bias += bf2f((uint16_t)((co & 1) ? (word >> 16) : (word & 0xFFFF)));
+      }
+    }
+
+    const int lrow = lane & 7, lm = lane >> 3;
+#pragma unroll 2
+    for (int p0 = 0; p0 < kGPix; p0 += 16) {
+      const int r = p0 >> lcols, xs = p0 & (cols - 1);
       // A = dZ^T (out channels x pixels) of both m-tiles
       uint32_t a[2][4];
 #pragma unroll
-      for (int m = 0; m < 2; ++m) {
-        const int px = xs + lrow + 8 * (lm >> 1);
-        ldsm_x4_t(smem_addr(&sm.dz[r][2 * m + (lm & 1)][px]), a[m][0], a[m][1], a[m][2], a[m][3]);
-      }
+      for (int m = 0; m < 2; ++m)
+        ldsm_x4_t(smem_addr(&sm.dz[2 * m + (lm & 1)][p0 + lrow + 8 * (lm >> 1)]), a[m][0], a[m][1], a[m][2], a[m][3]);
 #pragma unroll
       for (int k = 0; k < kMaxPairs; ++k) {
         if (k >= npairs) break;
         const int ky = ptap[k] / 3, kx = ptap[k] % 3;
         uint32_t b[4][2];
 #pragma unroll
-        for (int jp = 0; jp < 2; ++jp) {
-          const int px = xs + kx + lrow + 8 * (lm & 1);
-          ldsm_x4_t(smem_addr(&sm.a[r + ky][2 * jp + (lm >> 1)][px]), b[2 * jp][0], b[2 * jp][1],
-                    b[2 * jp + 1][0], b[2 * jp + 1][1]);
-        }
+        for (int jp = 0; jp < 2; ++jp)
+          ldsm_x4_t(smem_addr(&sm.a[2 * jp + (lm >> 1)][(r + ky) * inw + xs + kx + lrow + 8 * (lm & 1)]), b[2 * jp][0],
+                    b[2 * jp][1], b[2 * jp + 1][0], b[2 * jp + 1][1]);
         const uint32_t* am = a[pm[k]];
 #pragma unroll
         for (int j = 0; j < 4; ++j) mma_bf16(acc[k][j], am[0], am[1], am[2], am[3], b[j][0], b[j][1]);
       }
     }
   }
+  if (bias != 0.f) atomicAdd(db + (tid & 31), bias);
+  __syncthreads();
+  float* s_sum = reinterpret_cast<float*>(&sm);
   const int g = lane >> 2, t = lane & 3;
 #pragma unroll
   for (int k = 0; k < kMaxPairs; ++k) {
     if (k >= npairs) break;
-    const int tap = ptap[k];
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int co = 16 * pm[k] + g + 8 * (e >> 1), ci = 8 * j + 2 * t + (e & 1);
-        if (acc[k][j][e] != 0.f) atomicAdd(dW + (co * kC + ci) * 9 + tap, acc[k][j][e]);
+        s_sum[(co * kC + ci) * 9 + ptap[k]] = acc[k][j][e];
       }
+  }
+  __syncthreads();
+#pragma unroll 3
+  for (int i = tid; i < 9 * kC * kC / 4; i += 256) {
+    const float4 v = reinterpret_cast<const float4*>(s_sum)[i];
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dW + 4 * i), "f"(v.x), "f"(v.y), "f"(v.z),
+                 "f"(v.w)
+                 : "memory");
   }
 }
 
@@ -414,35 +436,94 @@ __global__ void embed_kernel(const uint4* __restrict__ Ft, uint32_t T, float* __
   G[i] = act_at(Ft, t, kTplDs, kTplDs, kCentre + (int)(o >> 1), kCentre + (int)(o & 1), (int)c);
 }
 
-// z[t][p] = alpha sum_o F(p + o) . G[t][o] for the P = n * H * W positions of
-// the crops (flat index ((k * H) + y) * W + x) and T <= 128 templates.
-constexpr int kHeadPos = 32;
-__global__ void __launch_bounds__(256) head_train_kernel(const uint4* __restrict__ F, uint32_t n, uint32_t H,
-                                                         uint32_t W, const float* __restrict__ G, uint32_t T,
-                                                         float* __restrict__ z) {
-  extern __shared__ float sh[];
-  float* s_f = sh;                          // [kHeadPos][kEmb + 1]
-  float* s_g = sh + kHeadPos * (kEmb + 1);  // [T][kEmb]
-  const size_t P = (size_t)n * H * W;
-  const size_t p0 = (size_t)blockIdx.x * kHeadPos;
-  for (int i = threadIdx.x; i < kHeadPos * kEmb; i += blockDim.x) {
-    const int pi = i / kEmb, k = i % kEmb, o = k / kC, c = k % kC;
-    const size_t p = p0 + pi;
-    float v = 0.f;
-    if (p < P) {
-      const uint32_t x = (uint32_t)(p % W), y = (uint32_t)((p / W) % H), k2 = (uint32_t)(p / ((size_t)W * H));
-      v = act_at(F, k2, H, W, (int)y + (o >> 1), (int)x + (o & 1), c);
-    }
-    s_f[pi * (kEmb + 1) + k] = v;
+// The three products of the training head are f32 (F and G hold bf16 values,
+// dz is f32 and stays so), on CUDA cores: 128 x 128 x P multiply-adds each, 33
+// us at the FP32 issue rate for P = 73728. Each is a register-tiled product
+// from shared memory (at least 8 multiply-adds per shared-memory wavefront);
+// one value per thread and step, as before, ran 310, 1480 and 410 us, these
+// 60, 95 and 62 us. z and dF keep their order of sums (one accumulator per
+// value, k ascending).
+
+// The 8 channels of unit u as floats.
+__device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
+  const uint32_t wd[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    f[2 * i] = __uint_as_float(wd[i] << 16);
+    f[2 * i + 1] = __uint_as_float(wd[i] & 0xFFFF0000u);
   }
-  for (int i = threadIdx.x; i < (int)T * kEmb; i += blockDim.x) s_g[i] = G[i];
-  __syncthreads();
-  const int pi = threadIdx.x & 31;
-  const size_t p = p0 + pi;
-  for (uint32_t t = threadIdx.x >> 5; t < T; t += blockDim.x >> 5) {
-    float s = 0.f;
-    for (int k = 0; k < kEmb; ++k) s = fmaf(s_f[pi * (kEmb + 1) + k], s_g[t * kEmb + k], s);
-    if (p < P) z[(size_t)t * P + p] = kAlpha * s;
+}
+
+// F at position p moved by offset o, channels 8 c .. 8 c + 7; zeros outside.
+__device__ __forceinline__ uint4 unit_at(const uint4* __restrict__ F, size_t p, size_t P, uint32_t H, uint32_t W,
+                                         uint32_t o, uint32_t c) {
+  if (p >= P) return make_uint4(0u, 0u, 0u, 0u);
+  const uint32_t hw = H * W, k = (uint32_t)(p / hw), r = (uint32_t)(p - (size_t)k * hw);
+  const uint32_t y = r / W + (o >> 1), x = r % W + (o & 1);
+  if (y >= H || x >= W) return make_uint4(0u, 0u, 0u, 0u);
+  return F[(((size_t)k * H + y) * kChunks + c) * W + x];
+}
+
+// z[t][p] = alpha sum_o F(p + o) . G[t][o] for the P = n * H * W positions of
+// the crops (flat index ((k * H) + y) * W + x) and T <= 128 templates. A block
+// keeps all templates in shared memory and goes through tiles of 64 positions;
+// a thread owns 8 templates x 4 positions.
+constexpr int kZPos = 64, kZPitch = kZPos + 4, kGPitch = 128 + 4;
+constexpr size_t kHeadSmem = sizeof(float) * kEmb * (kZPitch + kGPitch);
+__global__ void __launch_bounds__(256) head_train_kernel(const uint4* __restrict__ F, size_t P, uint32_t H, uint32_t W,
+                                                         const float* __restrict__ G, uint32_t T,
+                                                         float* __restrict__ z) {
+  extern __shared__ __align__(16) float sh[];
+  float* s_f = sh;                    // [kEmb][kZPitch]
+  float* s_g = sh + kEmb * kZPitch;   // [kEmb][kGPitch]
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  for (int i = threadIdx.x; i < kEmb * 128; i += 256) {
+    const int t = i / kEmb, k = i % kEmb;
+    s_g[k * kGPitch + t] = t < (int)T ? G[i] : 0.f;
+  }
+  const bool vec = P % 4 == 0;
+  for (size_t p0 = (size_t)blockIdx.x * kZPos; p0 < P; p0 += (size_t)gridDim.x * kZPos) {
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {  // 64 positions x 16 units
+      const int item = threadIdx.x + 256 * i, pi = item & 63, u = item >> 6;
+      float f[8];
+      unpack8(unit_at(F, p0 + pi, P, H, W, u >> 2, u & 3), f);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) s_f[(8 * u + e) * kZPitch + pi] = f[e];
+    }
+    __syncthreads();
+    float acc[8][4];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+#pragma unroll 4
+    for (int k = 0; k < kEmb; ++k) {
+      const float4 f = *reinterpret_cast<const float4*>(s_f + k * kZPitch + 4 * tx);
+      const float4 g0 = *reinterpret_cast<const float4*>(s_g + k * kGPitch + 8 * ty);
+      const float4 g1 = *reinterpret_cast<const float4*>(s_g + k * kGPitch + 8 * ty + 4);
+      const float fv[4] = {f.x, f.y, f.z, f.w}, gv[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(fv[j], gv[i], acc[i][j]);
+    }
+    const size_t p = p0 + 4 * tx;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const uint32_t t = 8 * ty + i;
+      if (t >= T || p >= P) continue;
+      float* o = z + (size_t)t * P + p;
+      if (vec) {
+        *reinterpret_cast<float4*>(o) =
+            make_float4(kAlpha * acc[i][0], kAlpha * acc[i][1], kAlpha * acc[i][2], kAlpha * acc[i][3]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (p + j < P) o[j] = kAlpha * acc[i][j];
+      }
+    }
   }
 }
 
@@ -465,7 +546,9 @@ __global__ void __launch_bounds__(1024) softmax_ce_kernel(float* __restrict__ z,
   __shared__ float s_lsen;
   float* zt = z + (size_t)blockIdx.x * P;
   float mx = -INFINITY;
-  for (size_t i = threadIdx.x; i < P; i += blockDim.x) mx = fmaxf(mx, zt[i]);
+  // eight loads in flight per thread in each of the three passes
+#pragma unroll 8
+  for (size_t i = threadIdx.x; i < P; i += 1024) mx = fmaxf(mx, zt[i]);
   for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = mx;
   __syncthreads();
@@ -478,7 +561,8 @@ __global__ void __launch_bounds__(1024) softmax_ce_kernel(float* __restrict__ z,
   mx = s_red[0];
   __syncthreads();
   float se = 0.f;
-  for (size_t i = threadIdx.x; i < P; i += blockDim.x) se += expf(zt[i] - mx);
+#pragma unroll 8
+  for (size_t i = threadIdx.x; i < P; i += 1024) se += expf(zt[i] - mx);
   for (int o = 16; o; o >>= 1) se += __shfl_xor_sync(0xffffffffu, se, o);
   if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = se;
   __syncthreads();
@@ -513,101 +597,136 @@ __global__ void __launch_bounds__(1024) softmax_ce_kernel(float* __restrict__ z,
   __syncthreads();
   const float lsen = s_lsen;
   const float inv = 1.0f / (float)T;
-  for (size_t i = threadIdx.x; i < P; i += blockDim.x) {
-    const float zi = zt[i];
+  // the positive's crop alone needs the neighbourhood's indices
+  const size_t hw = (size_t)H * W, crop = pos_ok ? (size_t)pt / hw * hw : P;
+  auto grad = [&](size_t i, float zi) {
     float d = expf(zi - lse);
-    if (pos_ok && in_nbhd(i, (size_t)pt, H, W)) d -= expf(zi - lsen);
+    if (i >= crop && i < crop + hw && in_nbhd(i, (size_t)pt, H, W)) d -= expf(zi - lsen);
     zt[i] = d * inv;
+  };
+  size_t i = threadIdx.x;
+  for (; i + 7 * 1024 < P; i += 8 * 1024) {
+    float v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = zt[i + k * 1024];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) grad(i + k * 1024, v[k]);
   }
+  for (; i < P; i += 1024) grad(i, zt[i]);
   if (threadIdx.x == 0) atomicAdd(loss, (lse - lsen) * inv);
 }
 
-// dF[q][c] = alpha sum_o sum_t dz[t][q - o] G[t][o][c] (bf16, row-chunked)
-__global__ void __launch_bounds__(256) head_grad_f_kernel(const float* __restrict__ dz, uint32_t n, uint32_t H,
+// dF[q][c] = alpha sum_o sum_t dz[t][q - o] G[t][o][c] (bf16, row-chunked). A
+// block owns 256 positions x 32 channels and goes through the offsets and
+// chunks of 32 templates; a thread owns 4 positions x 8 channels (one output
+// unit each), a warp 64 x 16.
+constexpr int kFPos = 256, kFPitch = kFPos + 4, kFTpl = 32;
+__global__ void __launch_bounds__(256) head_grad_f_kernel(const float* __restrict__ dz, size_t P, uint32_t H,
                                                           uint32_t W, const float* __restrict__ G, uint32_t T,
                                                           uint4* __restrict__ dF) {
-  extern __shared__ float sh[];
-  float* s_g = sh;                 // [T][kEmb]
-  float* s_dz = sh + T * kEmb;     // [4][kHeadPos][T]: dz at q - o
-  const size_t P = (size_t)n * H * W;
-  const size_t q0 = (size_t)blockIdx.x * kHeadPos;
-  for (int i = threadIdx.x; i < (int)T * kEmb; i += blockDim.x) s_g[i] = G[i];
-  for (int i = threadIdx.x; i < 4 * kHeadPos * (int)T; i += blockDim.x) {
-    const int t = i % T, qi = (i / T) % kHeadPos, o = i / (T * kHeadPos);
-    const size_t q = q0 + qi;
-    float v = 0.f;
-    if (q < P) {
-      const int x = (int)(q % W) - (o & 1), y = (int)((q / W) % H) - (o >> 1);
-      if (x >= 0 && y >= 0) v = dz[(size_t)t * P + (q - (o & 1) - (size_t)(o >> 1) * W)];
-    }
-    s_dz[i] = v;
-  }
-  __syncthreads();
-  // thread (q, chunk): 8 channels
-  const int qi = threadIdx.x >> 2, c8 = threadIdx.x & 3;
-  if (qi >= kHeadPos) return;
-  const size_t q = q0 + qi;
-  if (q >= P) return;
-  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  for (int o = 0; o < 4; ++o)
-    for (uint32_t t = 0; t < T; ++t) {
-      const float d = s_dz[(o * kHeadPos + qi) * T + t];
-      if (d == 0.f) continue;
-      const float* g = s_g + t * kEmb + o * kC + 8 * c8;
+  __shared__ __align__(16) float s_dz[kFTpl * kFPitch];  // dz at q - o
+  __shared__ __align__(16) float s_g[kFTpl * kC];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int ql = (warp & 3) * 64 + (lane & 15) * 4, chunk = (warp >> 2) * 2 + (lane >> 4);
+  const size_t q0 = (size_t)blockIdx.x * kFPos;
+  // the position whose gradients this thread stages
+  const size_t qs = q0 + threadIdx.x;
+  const uint32_t rs = (uint32_t)(qs % ((size_t)H * W)), ys = rs / W, xs = rs % W;
+  float acc[4][8];
 #pragma unroll
-      for (int e = 0; e < 8; ++e) acc[e] = fmaf(d, g[e], acc[e]);
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int e = 0; e < 8; ++e) acc[i][e] = 0.f;
+  for (uint32_t o = 0; o < 4; ++o) {
+    const bool in = qs < P && xs >= (o & 1) && ys >= (o >> 1);
+    const float* src = dz + (in ? qs - (o & 1) - (size_t)(o >> 1) * W : 0);
+    for (uint32_t t0 = 0; t0 < T; t0 += kFTpl) {
+      __syncthreads();
+#pragma unroll 16
+      for (uint32_t t = 0; t < kFTpl; ++t)
+        s_dz[t * kFPitch + threadIdx.x] = in && t0 + t < T ? src[(size_t)(t0 + t) * P] : 0.f;
+#pragma unroll
+      for (int i = 0; i < kFTpl * kC / 256; ++i) {
+        const uint32_t idx = threadIdx.x + 256 * i, t = idx / kC, c = idx % kC;
+        s_g[idx] = t0 + t < T ? G[(size_t)(t0 + t) * kEmb + o * kC + c] : 0.f;
+      }
+      __syncthreads();
+#pragma unroll 4
+      for (int t = 0; t < kFTpl; ++t) {
+        const float4 d = *reinterpret_cast<const float4*>(s_dz + t * kFPitch + ql);
+        const float4 g0 = *reinterpret_cast<const float4*>(s_g + t * kC + 8 * chunk);
+        const float4 g1 = *reinterpret_cast<const float4*>(s_g + t * kC + 8 * chunk + 4);
+        const float dv[4] = {d.x, d.y, d.z, d.w}, gv[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int e = 0; e < 8; ++e) acc[i][e] = fmaf(dv[i], gv[e], acc[i][e]);
+      }
     }
-  const uint32_t x = (uint32_t)(q % W), y = (uint32_t)((q / W) % H), k2 = (uint32_t)(q / ((size_t)W * H));
-  dF[(((size_t)k2 * H + y) * kChunks + c8) * W + x] =
-      make_uint4(pack2(kAlpha * acc[0], kAlpha * acc[1]), pack2(kAlpha * acc[2], kAlpha * acc[3]),
-                 pack2(kAlpha * acc[4], kAlpha * acc[5]), pack2(kAlpha * acc[6], kAlpha * acc[7]));
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const size_t q = q0 + ql + i;
+    if (q >= P) break;
+    const uint32_t x = (uint32_t)(q % W);
+    const size_t row = q / W;  // image and row
+    dF[(row * kChunks + chunk) * W + x] =
+        make_uint4(pack2(kAlpha * acc[i][0], kAlpha * acc[i][1]), pack2(kAlpha * acc[i][2], kAlpha * acc[i][3]),
+                   pack2(kAlpha * acc[i][4], kAlpha * acc[i][5]), pack2(kAlpha * acc[i][6], kAlpha * acc[i][7]));
+  }
 }
 
-// dG[t][k] += alpha sum_p dz[t][p] F4[p][k] over 256 positions per block
-constexpr int kGradPos = 256, kGradSub = 32;
-__global__ void __launch_bounds__(256) head_grad_g_kernel(const float* __restrict__ dz, const uint4* __restrict__ F,
-                                                          uint32_t n, uint32_t H, uint32_t W, uint32_t T,
-                                                          float* __restrict__ dG) {
-  extern __shared__ float sh[];
-  float* s_f = sh;                              // [kGradSub][kEmb]
-  float* s_d = sh + kGradSub * kEmb;            // [T][kGradSub]
-  const size_t P = (size_t)n * H * W;
-  const size_t p0 = (size_t)blockIdx.x * kGradPos;
-  // thread: output k = tid % 128, templates t = tid / 128, +2, ...
-  const int k = threadIdx.x % kEmb, t0 = threadIdx.x / kEmb;
-  float acc[64];
-  const int nt = ((int)T - t0 + 1) / 2;
+// dG[t][k] += alpha sum_p dz[t][p] F4[p][k], 256 positions per block (summed
+// in order, then one atomic per value); a thread owns 8 templates x 8 values.
+constexpr int kGradPos = 256, kGradSub = 32, kGradPitch = kGradSub + 4;
+__global__ void __launch_bounds__(256, 2) head_grad_g_kernel(const float* __restrict__ dz, const uint4* __restrict__ F,
+                                                             size_t P, uint32_t H, uint32_t W, uint32_t T,
+                                                             float* __restrict__ dG) {
+  __shared__ __align__(16) float s_f[kEmb * kGradPitch];
+  __shared__ __align__(16) float s_d[128 * kGradPitch];
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const size_t begin = (size_t)blockIdx.x * kGradPos, end = begin + kGradPos < P ? begin + kGradPos : P;
+  float acc[8][8];
 #pragma unroll
-  for (int i = 0; i < 64; ++i) acc[i] = 0.f;
-  for (int sub = 0; sub < kGradPos; sub += kGradSub) {
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+  for (size_t p0 = begin; p0 < end; p0 += kGradSub) {
     __syncthreads();
-    for (int i = threadIdx.x; i < kGradSub * kEmb; i += blockDim.x) {
-      const int pi = i / kEmb, kk = i % kEmb, o = kk / kC, c = kk % kC;
-      const size_t p = p0 + sub + pi;
-      float v = 0.f;
-      if (p < P) {
-        const uint32_t x = (uint32_t)(p % W), y = (uint32_t)((p / W) % H), k2 = (uint32_t)(p / ((size_t)W * H));
-        v = act_at(F, k2, H, W, (int)y + (o >> 1), (int)x + (o & 1), c);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {  // 32 positions x 16 units
+      const int u = warp + 8 * i;
+      float f[8];
+      unpack8(unit_at(F, p0 + lane, P, H, W, u >> 2, u & 3), f);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) s_f[(8 * u + e) * kGradPitch + lane] = f[e];
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const uint32_t t = warp + 8 * i;
+      s_d[t * kGradPitch + lane] = t < T && p0 + lane < P ? dz[(size_t)t * P + p0 + lane] : 0.f;
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int q = 0; q < kGradSub; q += 4) {
+      float4 f[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[j] = *reinterpret_cast<const float4*>(s_f + (tx + 16 * j) * kGradPitch + q);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float4 d = *reinterpret_cast<const float4*>(s_d + (ty + 16 * i) * kGradPitch + q);
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          acc[i][j] = fmaf(d.w, f[j].w, fmaf(d.z, f[j].z, fmaf(d.y, f[j].y, fmaf(d.x, f[j].x, acc[i][j]))));
       }
-      s_f[i] = v;
-    }
-    for (int i = threadIdx.x; i < (int)T * kGradSub; i += blockDim.x) {
-      const int t = i / kGradSub, pi = i % kGradSub;
-      const size_t p = p0 + sub + pi;
-      s_d[i] = p < P ? dz[(size_t)t * P + p] : 0.f;
-    }
-    __syncthreads();
-#pragma unroll 4
-    for (int pi = 0; pi < kGradSub; ++pi) {
-      const float f = s_f[pi * kEmb + k];
-#pragma unroll
-      for (int i = 0; i < 64; ++i)
-        if (i < nt) acc[i] = fmaf(s_d[(t0 + 2 * i) * kGradSub + pi], f, acc[i]);
     }
   }
 #pragma unroll
-  for (int i = 0; i < 64; ++i)
-    if (i < nt && acc[i] != 0.f) atomicAdd(dG + (size_t)(t0 + 2 * i) * kEmb + k, kAlpha * acc[i]);
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (ty + 16 * i < (int)T && acc[i][j] != 0.f)
+        atomicAdd(dG + (size_t)(ty + 16 * i) * kEmb + tx + 16 * j, kAlpha * acc[i][j]);
 }
 
 // dFt (templates' 12 x 12 feature gradient, bf16 row-chunked): dG at the 2x2 centre, 0 elsewhere
@@ -797,8 +916,10 @@ ipb_status trunk_backward(ipb_proposal_net* net, const uint8_t* img, uint32_t n,
   uint4* other = d1;
   for (int l = kLayers - 1; l >= 1; --l) {
     // weight gradient of layer l+1 (index l): dz x A_l
-    const dim3 grid((W + kTW - 1) / kTW, (H + kTH - 1) / kTH, n);
-    conv_grad_kernel<<<grid, 256, 0, s>>>(dz, acts[l - 1], H, W, net->grads + w_off(l), net->grads + b_off(l));
+    const uint32_t lcols = W > 32 ? 6 : W > 16 ? 5 : 4, cols = 1u << lcols, rows = kGPix / cols;
+    const uint32_t tx = (W + cols - 1) / cols, ty = (H + rows - 1) / rows, tiles = tx * ty * n;
+    conv_grad_kernel<<<std::min(tiles, 2u * (uint32_t)device_sm_count()), 256, 0, s>>>(
+        dz, acts[l - 1], H, W, lcols, tx, ty, tiles, net->grads + w_off(l), net->grads + b_off(l));
     count_launch(kKernelLearned);
     NET_CUDA(cudaGetLastError(), "weight gradient");
     // data gradient into A_l, times relu'(Z_l) = [A_l > 0]
@@ -849,29 +970,24 @@ ipb_status loss_and_grads(ipb_proposal_net* net, const uint8_t* scenes, uint32_t
                         net->tag),
            "template trunk");
   NET_CUDA(launch_embed(c.Ft, T, c.G, s), "embedding");
-  const size_t head_smem = sizeof(float) * (kHeadPos * (kEmb + 1) + T * kEmb);
-  const unsigned nblk = (unsigned)((P + kHeadPos - 1) / kHeadPos);
   static PerDeviceOnce attr;
   NET_CUDA(attr.run([] {
-             cudaError_t e = cudaFuncSetAttribute(head_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                  200 * 1024);
-             if (e == cudaSuccess)
-               e = cudaFuncSetAttribute(head_grad_f_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-             return e;
+             return cudaFuncSetAttribute(head_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)kHeadSmem);
            }),
            "kernel attributes");
-  head_train_kernel<<<nblk, 256, head_smem, s>>>(c.Fs, N, H, W, c.G, T, c.z);
+  const unsigned sms = (unsigned)device_sm_count();
+  const unsigned ztiles = (unsigned)((P + kZPos - 1) / kZPos);
+  head_train_kernel<<<std::min(ztiles, 2 * sms), 256, kHeadSmem, s>>>(c.Fs, P, H, W, c.G, T, c.z);
   count_launch(kKernelLearned);
   NET_CUDA(cudaGetLastError(), "head");
   softmax_ce_kernel<<<T, 1024, 0, s>>>(c.z, P, H, W, pos, T, c.loss);
   count_launch(kKernelLearned);
   NET_CUDA(cudaGetLastError(), "loss");
-  const size_t gf_smem = sizeof(float) * (T * kEmb + 4 * kHeadPos * T);
-  head_grad_f_kernel<<<nblk, 4 * kHeadPos, gf_smem, s>>>(c.z, N, H, W, c.G, T, c.d_a);
+  head_grad_f_kernel<<<(unsigned)((P + kFPos - 1) / kFPos), 256, 0, s>>>(c.z, P, H, W, c.G, T, c.d_a);
   count_launch(kKernelLearned);
   NET_CUDA(cudaGetLastError(), "head gradient (features)");
-  const size_t gg_smem = sizeof(float) * (kGradSub * kEmb + T * kGradSub);
-  head_grad_g_kernel<<<(unsigned)((P + kGradPos - 1) / kGradPos), 256, gg_smem, s>>>(c.z, c.Fs, N, H, W, T, c.dG);
+  head_grad_g_kernel<<<(unsigned)((P + kGradPos - 1) / kGradPos), 256, 0, s>>>(c.z, c.Fs, P, H, W, T, c.dG);
   count_launch(kKernelLearned);
   NET_CUDA(cudaGetLastError(), "head gradient (embedding)");
   const uint32_t tu = T * kTplDs * kChunks * kTplDs;
