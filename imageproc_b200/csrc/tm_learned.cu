@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(256) conv_mma_kernel(const uint4* __restrict__
 // over the 8 warps. A block goes through many tiles and adds its 9216 sums
 // once, staged in the gradient's order so that warps add contiguous 16-byte
 // runs. A block per tile with one scattered atomic per sum spent its time on
-// those: a layer of 128 crops of 24 x 24 135 us, now 22 us.
+// those: a layer of 128 crops of 24 x 24 135 us, now 30 us.
 constexpr int kGPix = 256;
 constexpr int kGIn = 18 * 18 > 10 * 34 ? (18 * 18 > 6 * 66 ? 18 * 18 : 6 * 66) : (10 * 34 > 6 * 66 ? 10 * 34 : 6 * 66);
 struct GradSmem {
@@ -441,7 +441,7 @@ __global__ void embed_kernel(const uint4* __restrict__ Ft, uint32_t T, float* __
 // us at the FP32 issue rate for P = 73728. Each is a register-tiled product
 // from shared memory (at least 8 multiply-adds per shared-memory wavefront);
 // one value per thread and step, as before, ran 310, 1480 and 410 us, these
-// 60, 95 and 62 us. z and dF keep their order of sums (one accumulator per
+// 70, 97 and 75 us. z and dF keep their order of sums (one accumulator per
 // value, k ascending).
 
 // The 8 channels of unit u as floats.
