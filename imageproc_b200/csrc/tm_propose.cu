@@ -53,7 +53,6 @@ constexpr int kWin = 32;          // verification window: 32 x 32 positions
 constexpr int kBlk = 12;          // certification block: 12 x 12 positions
 constexpr int kMaxExtra = 16384;  // most extra 4 x 4 blocks a template may verify
 constexpr int kVerifyCtas = 4 * 148;  // blocks of threads sharing all templates' extra blocks
-constexpr uint32_t kFallbackPerTemplate = 8;  // fallbacks up to this many use the single-template kernel
 constexpr int kPatch = kWin + kTpl - 1;        // 79 image rows / columns per window
 constexpr int kPatchPitch = 96;                // 16-byte multiple >= kPatch + 4
 
@@ -964,7 +963,6 @@ struct Carve {
   uint32_t* micro;
   uint32_t* span4;
   uint32_t* span16;
-  uint8_t* fb_tpl;
   unsigned long long* fb_keys;
   ipb_extremes_f32* fb_ext;
   size_t bytes;
@@ -1008,7 +1006,6 @@ Carve carve(uint8_t* base, uint32_t W, uint32_t H, uint32_t T, uint32_t k) {
   c.micro = reinterpret_cast<uint32_t*>(take((size_t)Mx * My * 4));
   c.span4 = reinterpret_cast<uint32_t*>(take((size_t)Mx * My * 4));
   c.span16 = reinterpret_cast<uint32_t*>(take((size_t)Mx * My * 4));
-  c.fb_tpl = reinterpret_cast<uint8_t*>(take((size_t)T * kTpl * kTpl));
   c.fb_keys = reinterpret_cast<unsigned long long*>(take((size_t)T * 16));
   c.fb_ext = reinterpret_cast<ipb_extremes_f32*>(take((size_t)T * sizeof(ipb_extremes_f32)));
   c.bytes = off;
@@ -1130,23 +1127,17 @@ ipb_status finish_queries(ProposeScratch& ps, const Carve& c, unsigned int call_
   if (!fb.empty()) {
     const uint32_t nf = (uint32_t)fb.size();
     P_CUDA(launch_many_keys_init(c.fb_keys, nf, s), "extremes init");
-    if (nf <= kFallbackPerTemplate) {
-      // a few templates: one single-template tensor-core launch over them
-      // (its cost grows with the templates; the many-templates kernel's
-      // hardly does below one block of templates)
-      const uint8_t* tp[kFallbackPerTemplate];
-      for (uint32_t i = 0; i < nf; ++i) tp[i] = d_templates + (size_t)fb[i] * kTpl * kTpl;
-      P_CUDA(launch_umma_extremes(d_image, W, H, tp, nf, kTpl, kTpl, IPB_SUM_OF_SQUARED_ERRORS,
-                                  IPB_PRECISION_EXACT_FP64, c.fb_keys, ps.err, call_tag, s),
-             "exhaustive fallback");
-    } else {
-      for (size_t i = 0; i < fb.size(); ++i)
-        P_CUDA(cudaMemcpyAsync(c.fb_tpl + i * kTpl * kTpl, d_templates + (size_t)fb[i] * kTpl * kTpl, kTpl * kTpl,
-                               cudaMemcpyDeviceToDevice, s),
-               "gather fallback templates");
-      P_CUDA(launch_many(d_image, W, H, c.fb_tpl, kTpl, kTpl, nf, IPB_SUM_OF_SQUARED_ERRORS,
-                         IPB_PRECISION_EXACT_FP64, nullptr, c.fb_keys, ps.err, call_tag, s, nullptr),
-             "exhaustive fallback");
+    // launches of up to eight templates without score maps, in sets that share
+    // the scene's staged tiles and window sums: about 0.13 ms a template at
+    // 8192 x 8192 (the many-templates kernel takes 11 ms for up to 16, 22 ms
+    // for 64)
+    for (uint32_t i0 = 0; i0 < nf; i0 += kInlineProblems) {
+      MatchArgs args[kInlineProblems];
+      const uint32_t n = std::min(kInlineProblems, nf - i0);
+      for (uint32_t i = 0; i < n; ++i)
+        args[i] = MatchArgs{d_image, W, H, d_templates + (size_t)fb[i0 + i] * kTpl * kTpl, kTpl, kTpl, nullptr, false,
+                            IPB_SUM_OF_SQUARED_ERRORS, IPB_PRECISION_EXACT_FP64, nullptr, s};
+      P_CUDA(launch_window_few(args, n, c.fb_keys + 2 * i0, ps.err, call_tag, s, nullptr), "exhaustive fallback");
     }
     P_CUDA(launch_many_keys_finish(c.fb_keys, Wo, c.fb_ext, nf, s), "extremes finish");
     P_CUDA(cudaMemcpyAsync(fb_ext.data(), c.fb_ext, sizeof(ipb_extremes_f32) * nf, cudaMemcpyDeviceToHost, s),

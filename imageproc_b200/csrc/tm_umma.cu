@@ -1019,36 +1019,6 @@ cudaError_t launch_umma_batch(const UmmaPlan& pl, UmmaLaunch& L, cudaStream_t st
   return e;
 }
 
-cudaError_t launch_umma_extremes(const uint8_t* img, uint32_t W, uint32_t H, const uint8_t* const* tpls,
-                                 uint32_t n, uint32_t w, uint32_t h, int method, int precision,
-                                 unsigned long long* keys, unsigned int* err_word, unsigned int tag,
-                                 cudaStream_t stream) {
-  if (n == 0) return cudaSuccess;
-  if (n > kInlineProblems || !umma_shape_ok(w, h, false)) return cudaErrorNotSupported;
-  // the templates share the image: sets of up to kMaxSet share its A rows
-  const uint32_t nsets = (n + kMaxSet - 1) / kMaxSet, set = (n + nsets - 1) / nsets;
-  UmmaPlan pl;
-  if (!make_plan(ks_of(w), false, h, /*tall=*/true, pl, 0, set) && !make_plan(ks_of(w), false, h, true, pl, 0, 1))
-    return cudaErrorNotSupported;
-  cudaError_t e = umma_prepare_kernels();
-  if (e != cudaSuccess) return e;
-  std::vector<UmmaProblem> probs;
-  for (uint32_t i = 0; i < n; ++i) {
-    const MatchArgs a{img, W, H, tpls[i], w, h, nullptr, false, method, precision, nullptr, stream};
-    probs.push_back(umma_problem(a, pl, 0, keys + 2 * i));
-  }
-  const uint32_t tiles = umma_make_sets(probs, pl);
-  UmmaLaunch L{};
-  for (uint32_t i = 0; i < n; ++i) L.inl[i] = probs[i];
-  L.nprobs = n;
-  L.tiles = tiles;
-  L.err = err_word;
-  L.tag = tag;
-  L.wait_ns = pipeline_wait_ns();
-  L.stall = pipeline_stall() ? 1u : 0u;
-  return launch_umma_batch(pl, L, stream, nullptr);
-}
-
 cudaError_t launch_umma(const MatchArgs& a, unsigned int* err_word, unsigned int tag) {
   UmmaPlan pl;
   if (!make_plan(ks_of(a.w), a.mask != nullptr, a.h, /*tall=*/false, pl)) return cudaErrorNotSupported;
