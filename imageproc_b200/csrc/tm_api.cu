@@ -194,7 +194,7 @@ struct Context {
   int device = -1;
   cudaStream_t stream = nullptr;
   cudaEvent_t last = nullptr;  // last use of any scratch buffer below
-  DevBuf scratch, ext_scratch, ext_result, img, tpl, mask, out;
+  DevBuf scratch, ext_scratch, img, tpl, mask, out;
   void* pinned = nullptr;  // small pinned host block: reduction results, error words
   DevBuf errw;                     // tensor-core error word (largest failing launch tag)
   DevBuf many_keys;                // per-template extremes keys of the many-templates path
@@ -242,7 +242,7 @@ struct Context {
     if (ostage) cudaFreeHost(ostage);
     for (cudaStream_t s : {s_in, s_out})
       if (s) cudaStreamDestroy(s);
-    for (DevBuf* b : {&scratch, &ext_scratch, &ext_result, &img, &tpl, &mask, &out, &errw, &many_keys, &rgb, &keys})
+    for (DevBuf* b : {&scratch, &ext_scratch, &img, &tpl, &mask, &out, &errw, &many_keys, &rgb, &keys})
       if (b->p) cudaFree(b->p);
     if (pinned) cudaFreeHost(pinned);
     if (last) cudaEventDestroy(last);
@@ -315,9 +315,10 @@ bool host_mask_is_binary(const uint8_t* m, size_t n) {
 // Synchronises the stream and reports a tensor-core wait that ran out in any
 // launch of this context since the last check (the error word holds the
 // largest failing launch tag; tags only grow).
-ipb_status finish_sync(Context* c, cudaStream_t s) {
+// err_copied: the error word is on its way to the pinned block already.
+ipb_status finish_sync(Context* c, cudaStream_t s, bool err_copied = false) {
   const bool check = c->tensor_since_check && c->errw.p;
-  if (check)
+  if (check && !err_copied)
     IPB_CUDA(cudaMemcpyAsync(static_cast<uint8_t*>(c->pinned) + 128, c->errw.p, sizeof(unsigned int),
                              cudaMemcpyDeviceToHost, s),
              "copy error word");
@@ -692,15 +693,16 @@ ipb_status extremes_common(Context* c, const T* d, uint32_t W, uint32_t H, R* ou
       typename std::conditional<std::is_same<T, int64_t>::value, long long, T>::type>::type;
   ipb_status st;
   if ((st = ensure(c, c->ext_scratch, extremes_scratch_bytes(), /*zero=*/true))) return st;
-  if ((st = ensure(c, c->ext_result, sizeof(ExtremesResult<DT>)))) return st;
   IPB_CUDA(cudaStreamWaitEvent(s, c->last, 0), "cudaStreamWaitEvent");
-  auto* res = static_cast<ExtremesResult<DT>*>(c->ext_result.p);
-  cudaError_t e = launch_find_extremes<DT>(reinterpret_cast<const DT*>(d), (unsigned long long)W * H,
-                                           c->ext_scratch.p, res, s);
+  // the kernel writes its record, and the tensor-core launches' error word,
+  // to the pinned block
+  const unsigned int* word = c->tensor_since_check ? static_cast<const unsigned int*>(c->errw.p) : nullptr;
+  cudaError_t e = launch_find_extremes<DT>(
+      reinterpret_cast<const DT*>(d), (unsigned long long)W * H, c->ext_scratch.p,
+      static_cast<ExtremesResult<DT>*>(c->pinned), s, word,
+      reinterpret_cast<unsigned int*>(static_cast<uint8_t*>(c->pinned) + 128));
   if (e != cudaSuccess) return cuda_fail(e, "find_extremes launch");
-  IPB_CUDA(cudaMemcpyAsync(c->pinned, res, sizeof(ExtremesResult<DT>), cudaMemcpyDeviceToHost, s),
-           "copy extremes");
-  if ((st = finish_sync(c, s))) return st;
+  if ((st = finish_sync(c, s, /*err_copied=*/word != nullptr))) return st;
   ExtremesResult<DT> r;
   std::memcpy(&r, c->pinned, sizeof(r));
   out->max_value = (T)r.max_value;

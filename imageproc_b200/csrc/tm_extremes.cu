@@ -10,9 +10,12 @@
 // index, which reproduces the scan's choice; NaNs are excluded from the
 // candidates and the seed rule is applied at the end.
 //
-// One launch: each block reduces a grid-stride share into a partial record;
-// the last block to finish (atomic ticket) reduces the partials, writes the
-// result and re-arms the ticket for the next call.
+// One launch: each block reduces a grid-stride share (eight loads in flight per
+// thread) into a partial record; the last block to finish (atomic ticket)
+// reduces the partials, writes the result and re-arms the ticket for the next
+// call. The result, and a word that the caller wants read with it, may go to
+// page-locked host memory: a call that waits for them needs no copies after
+// the kernel.
 #include <cfloat>
 #include <cmath>
 
@@ -23,7 +26,8 @@ namespace ipb {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kMaxBlocks = 148 * 8;
+constexpr int kMaxBlocks = 148 * 4;
+constexpr int kInFlight = 8;  // loads per thread
 
 template <typename T>
 __device__ __forceinline__ bool is_nan(T v) {
@@ -88,7 +92,8 @@ template <typename T>
 __global__ void __launch_bounds__(kThreads)
 extremes_kernel(const T* __restrict__ data, unsigned long long n,
                 Cand<typename Wide<T>::type>* __restrict__ partials, unsigned int* __restrict__ ticket,
-                ExtremesResult<T>* __restrict__ result) {
+                ExtremesResult<T>* __restrict__ result, const unsigned int* __restrict__ word,
+                unsigned int* __restrict__ word_out) {
   using V = typename Wide<T>::type;
   using C = Cand<V>;
   __shared__ C s_warp[kThreads / 32];
@@ -98,9 +103,8 @@ extremes_kernel(const T* __restrict__ data, unsigned long long n,
   c.mn = c.mx = V(0);
   c.imn = c.imx = 0;
   const unsigned long long stride = (unsigned long long)gridDim.x * kThreads;
-  for (unsigned long long k = (unsigned long long)blockIdx.x * kThreads + threadIdx.x; k < n; k += stride) {
-    const T v = data[k];
-    if (is_nan(v)) continue;
+  auto take = [&](T v, unsigned long long k) {
+    if (is_nan(v)) return;
     const V wv = (V)v;
     if (!c.has) {
       c.mn = c.mx = wv;
@@ -110,7 +114,17 @@ extremes_kernel(const T* __restrict__ data, unsigned long long n,
       if (wv < c.mn) { c.mn = wv; c.imn = k; }  // increasing k: strict keeps the first
       if (wv > c.mx) { c.mx = wv; c.imx = k; }
     }
+  };
+  // eight loads in flight per thread
+  unsigned long long k = (unsigned long long)blockIdx.x * kThreads + threadIdx.x;
+  for (; k + (kInFlight - 1) * stride < n; k += kInFlight * stride) {
+    T v[kInFlight];
+#pragma unroll
+    for (int i = 0; i < kInFlight; ++i) v[i] = data[k + i * stride];
+#pragma unroll
+    for (int i = 0; i < kInFlight; ++i) take(v[i], k + i * stride);
   }
+  for (; k < n; k += stride) take(data[k], k);
   c = block_reduce(c, s_warp);
   if (threadIdx.x == 0) {
     partials[blockIdx.x] = c;
@@ -151,6 +165,7 @@ extremes_kernel(const T* __restrict__ data, unsigned long long n,
       r.min_index = acc.imn;
     }
     *result = r;
+    if (word) *word_out = __ldcg(word);
     *ticket = 0u;  // re-arm for the next launch on this scratch
   }
 }
@@ -163,8 +178,8 @@ size_t extremes_scratch_bytes() {
 }
 
 template <typename T>
-cudaError_t launch_find_extremes(const T* d, unsigned long long n, void* scratch,
-                                 ExtremesResult<T>* d_result, cudaStream_t s) {
+cudaError_t launch_find_extremes(const T* d, unsigned long long n, void* scratch, ExtremesResult<T>* result,
+                                 cudaStream_t s, const unsigned int* word, unsigned int* word_out) {
   using C = Cand<typename Wide<T>::type>;
   uint8_t* base = static_cast<uint8_t*>(scratch);
   C* partials = reinterpret_cast<C*>(base);
@@ -173,7 +188,7 @@ cudaError_t launch_find_extremes(const T* d, unsigned long long n, void* scratch
   unsigned long long blocks = (n + kThreads * 8 - 1) / (kThreads * 8);
   if (blocks < 1) blocks = 1;
   if (blocks > (unsigned long long)kMaxBlocks) blocks = kMaxBlocks;
-  extremes_kernel<T><<<(unsigned)blocks, kThreads, 0, s>>>(d, n, partials, ticket, d_result);
+  extremes_kernel<T><<<(unsigned)blocks, kThreads, 0, s>>>(d, n, partials, ticket, result, word, word_out);
   count_launch(kKernelExtremes);
   return cudaGetLastError();
 }
@@ -202,7 +217,8 @@ cudaError_t launch_extremes_to_struct(const ExtremesResult<float>* r, uint32_t w
 
 #define IPB_INSTANTIATE_EXTREMES(T)                                                            \
   template cudaError_t launch_find_extremes<T>(const T*, unsigned long long, void*,            \
-                                               ExtremesResult<T>*, cudaStream_t);
+                                               ExtremesResult<T>*, cudaStream_t, const unsigned int*, \
+                                               unsigned int*);
 IPB_INSTANTIATE_EXTREMES(uint8_t)
 IPB_INSTANTIATE_EXTREMES(uint16_t)
 IPB_INSTANTIATE_EXTREMES(uint32_t)

@@ -366,7 +366,7 @@ size_t reference_scratch_bytes(const MatchArgs& a);
 cudaError_t launch_reference(const MatchArgs& a, void* scratch);
 
 // ---- find_extremes (tm_extremes.cu) ----------------------------------------
-// Result record written to device memory by the reduction.
+// Result record written by the reduction, to device or page-locked host memory.
 template <typename T>
 struct ExtremesResult {
   T max_value;
@@ -376,8 +376,9 @@ struct ExtremesResult {
 };
 size_t extremes_scratch_bytes();
 template <typename T>
-cudaError_t launch_find_extremes(const T* d, unsigned long long n, void* scratch,
-                                 ExtremesResult<T>* d_result, cudaStream_t s);
+cudaError_t launch_find_extremes(const T* d, unsigned long long n, void* scratch, ExtremesResult<T>* result,
+                                 cudaStream_t s, const unsigned int* word = nullptr,
+                                 unsigned int* word_out = nullptr);  // *word_out = *word, beside the result
 // ExtremesResult<float> of a map of the given width -> ipb_extremes_f32 (device)
 cudaError_t launch_extremes_to_struct(const ExtremesResult<float>* r, uint32_t width, ipb_extremes_f32* out,
                                       cudaStream_t s);
