@@ -303,7 +303,7 @@ struct WindowProblem {
   uint32_t W, H, w, h;
   uint32_t Wo, Ho, tiles_x, tile_begin;  // tile_begin: first global tile of the problem
   uint32_t K, pitch;        // bytes per template-block row (w + 15 rounded up to 32), staged image row pitch
-  uint32_t nch, crows;      // chunks of template rows, rows per chunk
+  uint32_t nch, csteps, both;  // chunks of MMA steps, steps per chunk, whether one chunk takes both block slots
   uint32_t load_mode, tile_bytes;
   int method, precision;
   // members of the set this problem leads (0 on the others, which follow it);

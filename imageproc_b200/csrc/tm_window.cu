@@ -1,6 +1,6 @@
 // tm_window.cu -- exact template matching on the 5th-generation tensor cores
-// with the staged image tile itself as the MMA's A operand (tcgen05.mma
-// kind::i8, unsigned u8 x u8 -> s32, accumulators in tensor memory).
+// with the staged image tile itself as an MMA operand (tcgen05.mma kind::i8,
+// unsigned u8 x u8 -> s32, accumulators in tensor memory).
 //
 // Replaces the scalar walk of methods::*::score_at (src/template_matching.rs:
 // 219-376) for unmasked and binary-masked matches with templates up to
@@ -9,29 +9,35 @@
 // fused into the epilogue.
 //
 // Formulation. A tile is 128 output columns by 16 NJ output rows (NJ = 1, 2,
-// 4 or 8). Tensor-memory lane m = 8 G + c (G = 0..15, c = 0..7) stands for
-// the output columns x0 + 16 c + s (s = 0..15) of the output rows y0 + NJ G +
-// j (j = 0..NJ-1); the accumulator column of (j, s) is 16 j + s. For every
-// step rho = 0 .. NJ + h - 2 and K step kk (32 bytes):
-//   A_rho[8 G + c][k] = I[y0 + NJ G + rho][x0 + 16 c + k]            k < K
-//   B_rho[(j, s)][k]  = T[rho - j][k - s]  (0 <= k - s < w, 0 <= rho - j < h)
-//   D[m][(j, s)] += sum_k A_rho[m][k] B_rho[(j, s)][k]
-// with K = w + 15 rounded up to 32, so that D[m][(j, s)] is the correlation X
-// at its output position. A needs no building: in the canonical no-swizzle
-// K-major layout a core matrix is eight 16-byte rows, 16 bytes apart, and the
-// tile of image rows staged with a pitch of P >= 127 + w bytes is read in
-// place: lanes 16 bytes apart are the overlapping windows of one image row,
-// 16 bytes between the two K halves (LBO), NJ P bytes between 8-lane groups
-// (SBO), and step rho starts rho rows further down. The whole tile is resident,
-// so no step waits for data. B is a window of one buffer: the template rows'
-// 16-shift blocks (16 rows of K bytes each) in decreasing template row, so
-// the blocks of the output rows that a step feeds are consecutive and the
-// MMA's N is 16 times their number.
+// 4 or 8). Tensor-memory lane m = 16 j + s (j = 0..7, s = 0..15) and
+// accumulator column n = 8 G + c (G = 0..2NJ-1, c = 0..7) stand for the output
+// at row y0 + 8 G + j, column x0 + 16 c + s. For every step rho = 0 .. h + 6
+// and K step kk (32 bytes):
+//   A_rho[(j, s)][k]  = T[rho - j][k - s]  (0 where outside the template)
+//   B_rho[8 G + c][k] = I[y0 + 8 G + rho][x0 + 16 c + k]             k < K
+//   D[m][n] += sum_k A_rho[m][k] B_rho[n][k]
+// with K = w + 15 rounded up to 32, so that D[m][n] is the correlation X at
+// its output position. B needs no building: in the canonical no-swizzle
+// K-major layout a core matrix is eight 16-byte rows, and the tile of image
+// rows staged with a pitch of P >= 127 + w bytes is read in place: rows n 16
+// bytes apart are the overlapping windows of one image row, 16 bytes between
+// the two K halves (LBO), 8 P bytes between 8-row groups (SBO), and step rho
+// starts rho rows further down. The whole tile is resident, so no step waits
+// for data. A is a window of one buffer: the template rows' 16-shift blocks
+// (16 rows of K bytes each) in decreasing template row, with zero blocks on
+// both sides; moving to the next step moves A's start back by one block.
 //
 // Against the Hankel-row kernel (tm_umma.cu), which forms every image row's A
 // operand with builder warps and hands stages of rows to the MMA warp, the
 // tensor pipe runs a whole tile without a hand-off; it pays K / w in extra
-// MACs (1.5 at w = 64) where that kernel pays its 16-row bands.
+// MACs (1.5 at w = 64) where that kernel pays its 16-row bands. What is short
+// then is shared memory: an MMA of 128 x 128 x 32 reads 8 KB of operands in 64
+// cycles, all the bandwidth there is, so every other access delays the tile.
+// Hence the lanes stand for (row, shift): sixteen lanes hold sixteen
+// neighbouring columns, and scores go from registers to the map without
+// staging (with lanes for 16-column groups, scores were transposed through
+// shared memory: four unmasked 1080p maps with 64 x 64 templates 65 us, so
+// 56 us).
 //
 //   unmasked:     X from I and T; the window sums Y = sum I^2 are formed from
 //                 the staged tile by the workers beside the MMAs (column
@@ -99,6 +105,7 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
 template <int kCount>
 __device__ __forceinline__ bool bar_or(uint32_t id, bool fail) {
   uint32_t r;
+  __syncwarp();
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.u32 p, %1, 0;\n\t"
@@ -172,18 +179,19 @@ struct BlockState {
   const uint8_t* tpl = nullptr;
   const uint8_t* mask = nullptr;
   uint32_t w = 0, h = 0, first = 0, nch = 0;
-  bool with_mask = false;  // the mask's blocks lie beside the template's
-  // moves on to q's template; true when all its blocks are still in the slots
-  __device__ __forceinline__ bool enter(const WindowProblem& q, bool need_mask) {
-    if (nch && nch <= 2 && tpl == q.tpl && mask == q.mask && w == q.w && h == q.h && (with_mask || !need_mask))
+  bool mask_last = false;  // the mask's blocks followed the template's
+  // moves on to q's template (with_y: and its mask); true when all its blocks
+  // are still in the slots
+  __device__ __forceinline__ bool enter(const WindowProblem& q, bool with_y) {
+    if (nch && nch <= 2 && !mask_last && !with_y && tpl == q.tpl && mask == q.mask && w == q.w && h == q.h)
       return true;
-    first = (first + nch) & 1u;
-    nch = q.nch;
+    first = q.both ? 0u : (first + nch) & 1u;
+    nch = (q.both ? 2u : q.nch) * (with_y ? 2u : 1u);  // a chunk over both slots uses each once
     tpl = q.tpl;
     mask = q.mask;
     w = q.w;
     h = q.h;
-    with_mask = need_mask;
+    mask_last = with_y;
     return false;
   }
 };
@@ -234,10 +242,14 @@ __device__ __forceinline__ void load_image(const WindowProblem& q, const Walk& w
 }
 
 // The same as one tensor copy (rows and columns past the image are zeros),
-// issued by one thread and counted on `bar`, its arrival included.
-__device__ __forceinline__ void load_tensor(const CUtensorMap* map, const Walk& w, uint8_t* dst, uint32_t bytes,
-                                            uint64_t* bar) {
+// issued by one thread, which makes all of the phase's arrivals on `bar`: no
+// arrival for a phase may precede the last phase's bytes. A map in global
+// memory was written by the host: the fence orders its reads after that.
+__device__ __forceinline__ void load_tensor(const CUtensorMap* map, bool global, const Walk& w, uint8_t* dst,
+                                            uint32_t bytes, uint64_t* bar) {
+  if (global) asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(map) : "memory");
   mbar_arrive_expect_tx(bar, bytes);
+  for (uint32_t i = 1; i < kLoadWarps; ++i) mbar_arrive(bar);
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::
           "r"(smem_u32(dst)),
@@ -284,15 +296,17 @@ __device__ __forceinline__ void add_tss(const uint8_t* raw, uint32_t pixels, uin
   if ((t & 31u) == 0) atomicAdd(tss, t2);
 }
 
-// The 16-shift blocks of template rows [d0, d0 + n), in decreasing row: block
-// b holds rows s = 0..15 of K bytes, byte k = T[d0 + n - 1 - b][k - s] (0
-// outside the row), in the canonical no-swizzle K-major layout (s / 8) 8K +
-// (k / 16) 128 + (s % 8) 16. A warp writes four core matrices (512 bytes) of a
-// row at once; the K / 32 such groups of all rows are shared out over `nw`
-// warps group by group, so that a lane mostly keeps its shift, its chunk and
-// the bytes of it that lie in the row while it goes down the rows.
-__device__ __forceinline__ void build_blocks(uint32_t K, uint32_t w, uint32_t d0, uint32_t n, const uint8_t* raw,
-                                             uint8_t* dst, uint32_t iw, uint32_t nw, uint32_t lane) {
+// The 16-shift blocks of n consecutive template rows in decreasing order from
+// row `top` (rows outside the template are zero): block b holds rows s = 0..15
+// of K bytes, byte k = T[top - b][k - s] (0 outside the row), in the canonical
+// no-swizzle K-major layout (s / 8) 8K + (k / 16) 128 + (s % 8) 16. A warp
+// writes four core matrices (512 bytes) of a row at once; the K / 32 such
+// groups of all rows are shared out over `nw` warps group by group, so that a
+// lane mostly keeps its shift, its chunk and the bytes of it that lie in the
+// row while it goes down the rows.
+__device__ __forceinline__ void build_blocks(uint32_t K, uint32_t w, uint32_t h, uint32_t top, uint32_t n,
+                                             const uint8_t* raw, uint8_t* dst, uint32_t iw, uint32_t nw,
+                                             uint32_t lane) {
   const uint32_t cpr = K / 16, items = (K / 32) * n;
   uint32_t item = iw * items / nw;
   const uint32_t end = (iw + 1) * items / nw;
@@ -312,10 +326,12 @@ __device__ __forceinline__ void build_blocks(uint32_t K, uint32_t w, uint32_t d0
     const uint32_t first = 16 + 16 * ch - sft;  // sixteen bytes of slack lie ahead of the template
     // four rows' reads ahead of their stores
     for (uint32_t b0 = item - grp * n; b0 < b_end; b0 += 4) {
-      uint32_t wd[4][5], sel[4];
+      uint32_t wd[4][5], sel[4], ok[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const uint32_t at = first + (d0 + n - 1 - min(b0 + i, n - 1)) * w;
+        const uint32_t d = top - (b0 + i);  // wraps below row 0
+        ok[i] = d < h ? 0xFFFFFFFFu : 0u;
+        const uint32_t at = first + (d < h ? d : 0u) * w;
         const uint32_t* a4 = reinterpret_cast<const uint32_t*>(raw - 16 + (at & ~3u));
         sel[i] = 0x3210u + (at & 3u) * 0x1111u;
 #pragma unroll
@@ -325,24 +341,24 @@ __device__ __forceinline__ void build_blocks(uint32_t K, uint32_t w, uint32_t d0
       for (int i = 0; i < 4; ++i)
         if (b0 + i < b_end)
           *reinterpret_cast<uint4*>(out + (b0 + i) * 16 * K) =
-              make_uint4(__byte_perm(wd[i][0], wd[i][1], sel[i]) & mask[0],
-                         __byte_perm(wd[i][1], wd[i][2], sel[i]) & mask[1],
-                         __byte_perm(wd[i][2], wd[i][3], sel[i]) & mask[2],
-                         __byte_perm(wd[i][3], wd[i][4], sel[i]) & mask[3]);
+              make_uint4(__byte_perm(wd[i][0], wd[i][1], sel[i]) & mask[0] & ok[i],
+                         __byte_perm(wd[i][1], wd[i][2], sel[i]) & mask[1] & ok[i],
+                         __byte_perm(wd[i][2], wd[i][3], sel[i]) & mask[2] & ok[i],
+                         __byte_perm(wd[i][3], wd[i][4], sel[i]) & mask[3] & ok[i]);
     }
     item = grp * n + b_end;
   }
 }
 
-// One chunk of the problem's template (and, masked, of the mask) into a slot.
-template <bool MASKED>
-__device__ __forceinline__ void build_chunk(const WindowProblem& q, uint32_t c, const uint8_t* raw,
-                                            uint32_t raw_bytes, uint8_t* slot, bool with_mask, uint32_t iw,
-                                            uint32_t nw, uint32_t lane) {
-  const uint32_t d0 = c * q.crows, n = min(q.crows, q.h - d0);
-  build_blocks(q.K, q.w, d0, n, raw, slot, iw, nw, lane);
-  if (MASKED && with_mask)
-    build_blocks(q.K, q.w, d0, n, raw + raw_bytes, slot + q.crows * 16 * q.K, iw, nw, lane);
+// Chunk cc of a problem: the blocks of template rows r1 - 1 down to r0 - 7 for
+// its steps [r0, r1); the template's chunks first, then (masked sets that need
+// window sums) the mask's.
+__device__ __forceinline__ void build_chunk(const WindowProblem& q, uint32_t cc, const uint8_t* raw,
+                                            uint32_t raw_bytes, uint8_t* slot, uint32_t iw, uint32_t nw,
+                                            uint32_t lane) {
+  const uint32_t c = cc < q.nch ? cc : cc - q.nch;
+  const uint32_t r0 = c * q.csteps, r1 = min(r0 + q.csteps, q.h + 7);
+  build_blocks(q.K, q.w, q.h, r1 - 1, r1 - r0 + 7, cc < q.nch ? raw : raw + raw_bytes, slot, iw, nw, lane);
 }
 
 __device__ __forceinline__ void add_squares(uint2 v, uint32_t (&a)[8]) {
@@ -377,10 +393,12 @@ __device__ __forceinline__ void add_squares4(uint2 r0, uint2 r1, uint2 r2, uint2
   }
 }
 
-// 16-byte chunk of a 128-word row, permuted so that lanes that own runs of 16
-// words, lanes that own runs of 8 and lanes that own single words all reach
-// different banks.
-__device__ __forceinline__ uint32_t chunk_at(uint32_t cc) { return cc ^ ((cc >> 3) & 3u); }
+// Word of the window sum at (row, x) of the tile: odd rows have the halves of
+// each 32-word run swapped, so that the sixteen lanes that read one row and
+// the sixteen that read the next reach different banks.
+__device__ __forceinline__ uint32_t sum_at(uint32_t row, uint32_t x) {
+  return row * kTileW + (x ^ ((row & 1u) << 4));
+}
 
 // Window sums Y = sum I^2 of `nr` output rows from tile row `row0` (one warp):
 // a lane owns eight image columns, keeps their sums over h rows (one row added
@@ -443,13 +461,13 @@ __device__ __forceinline__ void window_sums(const uint8_t* img, uint32_t pitch, 
       y1[k] = __shfl_sync(0xffffffffu, q1[(k + B) & 7], from) - q1[k];
     }
     if (lane < 16) {
-      uint4* row = reinterpret_cast<uint4*>(ytile + (row0 + i) * kTileW);
-      row[chunk_at(2 * lane)] = make_uint4(y0[0], y0[1], y0[2], y0[3]);
-      row[chunk_at(2 * lane + 1)] = make_uint4(y0[4], y0[5], y0[6], y0[7]);
+      uint4* row = reinterpret_cast<uint4*>(ytile + sum_at(row0 + i, 8 * lane));
+      row[0] = make_uint4(y0[0], y0[1], y0[2], y0[3]);
+      row[1] = make_uint4(y0[4], y0[5], y0[6], y0[7]);
       if (two) {
-        row += kTileW / 4;
-        row[chunk_at(2 * lane)] = make_uint4(y1[0], y1[1], y1[2], y1[3]);
-        row[chunk_at(2 * lane + 1)] = make_uint4(y1[4], y1[5], y1[6], y1[7]);
+        row = reinterpret_cast<uint4*>(ytile + sum_at(row0 + i + 1, 8 * lane));
+        row[0] = make_uint4(y1[0], y1[1], y1[2], y1[3]);
+        row[1] = make_uint4(y1[4], y1[5], y1[6], y1[7]);
       }
     }
     if (i + 2 < nr) {
@@ -489,33 +507,27 @@ __device__ __forceinline__ void square_planes(uint32_t v, uint32_t& lo, uint32_t
   hi = __byte_perm(p01, p23, 0x7632);
 }
 
-// One worker warp's share of a tile's epilogue: lane quadrant `quad` (lane
-// groups 4 quad .. + 3), rows j0 .. j1 - 1 of each group.
+// One worker warp's share of a tile's epilogue: lane quadrant `quad` (rows j =
+// 2 quad and 2 quad + 1 of every group), groups g0 .. g1 - 1 of eight rows.
 struct Epi {
   const WindowProblem& q;
   const Walk& w;
-  uint32_t nj, acc, accw;  // tensor-memory address (lane quadrant, buffer), columns per accumulator
-  uint32_t quad, lane, j0, j1, tss;
-  double td, tc;    // TSS and -2^52 TSS
-  uint32_t* ytile;  // window sums; each row's place also stages its scores
-  bool keep;        // the set's later members need the window sums
+  uint32_t acc;  // tensor-memory address (lane quadrant, buffer)
+  uint32_t j, s, lane, g0, g1, tss;  // j, s: the lane's row of a group and shift
+  double td, tc;                     // TSS and -2^52 TSS
+  uint32_t* ytile;
 };
 
 // Masked: the warp's window sums Y = 256 Dhi + Dlo from the accumulators at
-// `acc` (then accw columns further) into the tile.
-__device__ __forceinline__ void gather_sums(const Epi& e, uint32_t acc) {
-  const uint32_t g = e.lane >> 3, c = e.lane & 7u;
-  for (uint32_t j = e.j0; j < e.j1; ++j) {
-    uint4* mine = reinterpret_cast<uint4*>(e.ytile + (e.nj * (4 * e.quad + g) + j) * kTileW);
-    uint32_t lo[16], hi[16];
-    tmem_ld16(acc + 16 * j, lo);
-    tmem_ld16(acc + e.accw + 16 * j, hi);
+// `lo` and `hi` into the tile.
+__device__ __forceinline__ void gather_sums(const Epi& e, uint32_t lo, uint32_t hi) {
+  for (uint32_t g = e.g0; g < e.g1; ++g) {
+    uint32_t a[8], b[8];
+    tmem_ld8(lo + 8 * g, a);
+    tmem_ld8(hi + 8 * g, b);
     tmem_wait_ld();
 #pragma unroll
-    for (int k = 0; k < 16; ++k) lo[k] += 256u * hi[k];
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-      mine[chunk_at(4 * c + k)] = make_uint4(lo[4 * k], lo[4 * k + 1], lo[4 * k + 2], lo[4 * k + 3]);
+    for (uint32_t c = 0; c < 8; ++c) e.ytile[sum_at(8 * g + e.j, 16 * c + e.s)] = a[c] + 256u * b[c];
   }
 }
 
@@ -524,102 +536,70 @@ __device__ __forceinline__ void epilogue(const Epi& e) {
   constexpr bool kNeedY = kMethod != kCcorr;
   constexpr bool kFilter = method_is_norm(kMethod) && kFp64;
   const WindowProblem& q = e.q;
-  const uint32_t g = e.lane >> 3, c = e.lane & 7u;
-  const uint32_t xl = e.w.x0 + 16 * c;              // the lane's first column
-  const uint32_t gy0 = e.w.y0 + e.nj * 4 * e.quad;  // the quadrant's first row
+  const uint32_t x0 = e.w.x0 + e.s;  // the lane's first column; the others 16 further each
+  const uint32_t nv = x0 < q.Wo ? min(8u, (q.Wo - x0 + 15) / 16) : 0u;  // columns inside the map
   unsigned long long kmin = ~0ull, kmax = 0ull;
-  for (uint32_t j = e.j0; j < e.j1; ++j) {
-    if (gy0 + j >= q.Ho) break;  // warp-uniform: the lowest group's row
-    uint4* mine = reinterpret_cast<uint4*>(e.ytile + (e.nj * (4 * e.quad + g) + j) * kTileW);
-    const uint32_t y = gy0 + e.nj * g + j;
-    const uint32_t nv = y < q.Ho && xl < q.Wo ? min(16u, q.Wo - xl) : 0u;  // the lane's scores inside the map
-    uint32_t mn = 0xFFFFFFFFu, jmn = 0, mx = 0u, jmx = 0;
-    uint4 ys[4];
+  for (uint32_t g = e.g0; g < e.g1; ++g) {
+    if (e.w.y0 + 8 * g >= q.Ho) break;  // the group's first row
+    uint32_t x[8], yw[8];
+    tmem_ld8(e.acc + 8 * g, x);
+    if constexpr (kNeedY) {
 #pragma unroll
-    for (int hf = 0; hf < 2; ++hf) {
-      uint32_t x[8], yw[8];
-      tmem_ld8(e.acc + 16 * j + 8 * hf, x);
-      const uint32_t at0 = chunk_at(4 * c + 2 * hf), at1 = chunk_at(4 * c + 2 * hf + 1);
-      if constexpr (kNeedY) {
-        const uint4 v0 = mine[at0], v1 = mine[at1];
-        ys[2 * hf] = v0;
-        ys[2 * hf + 1] = v1;
-        yw[0] = v0.x, yw[1] = v0.y, yw[2] = v0.z, yw[3] = v0.w;
-        yw[4] = v1.x, yw[5] = v1.y, yw[6] = v1.z, yw[7] = v1.w;
-      } else if (e.keep) {
-        ys[2 * hf] = mine[at0];
-        ys[2 * hf + 1] = mine[at1];
+      for (uint32_t c = 0; c < 8; ++c) yw[c] = e.ytile[sum_at(8 * g + e.j, 16 * c + e.s)];
+    }
+    tmem_wait_ld();
+    uint32_t b[8];
+    if constexpr (kFilter) {
+      // every score through the filter, as independent chains; if any is
+      // undecided (rare), the lane's eight again, exactly
+      bool again = e.tss == 0;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const uint32_t score = method_is_sse(kMethod) ? yw[k] + e.tss - 2u * x[k] : x[k];
+        b[k] = norm_bits_fp64_filter(score, yw[k], e.td, e.tc, again);
       }
-      tmem_wait_ld();
-      uint32_t b[8];
-      if constexpr (kFilter) {
-        // every score through the filter, as independent chains; if any is
-        // undecided (rare), the lane's eight again, exactly
-        bool again = e.tss == 0;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const uint32_t score = method_is_sse(kMethod) ? yw[k] + e.tss - 2u * x[k] : x[k];
-          b[k] = norm_bits_fp64_filter(score, yw[k], e.td, e.tc, again);
-        }
-        if (again) {
-#pragma unroll
-          for (int k = 0; k < 8; ++k)
-            b[k] = __float_as_uint(finish_score32(kMethod, IPB_PRECISION_EXACT_FP64, x[k], yw[k], e.tss));
-        }
-      } else {
+      if (again) {
 #pragma unroll
         for (int k = 0; k < 8; ++k)
-          b[k] = __float_as_uint(finish_score32(kMethod, kFp64 ? IPB_PRECISION_EXACT_FP64 : IPB_PRECISION_EXACT_F32,
-                                                x[k], kNeedY ? yw[k] : 0u, e.tss));
+          b[k] = __float_as_uint(finish_score32(kMethod, IPB_PRECISION_EXACT_FP64, x[k], yw[k], e.tss));
       }
-      if constexpr (kExt) {
-        // scores are never negative, so their f32 bits order like the values;
-        // strict comparisons keep the first occurrence
+    } else {
 #pragma unroll
-        for (int k = 0; k < 8; ++k)
-          if ((uint32_t)(8 * hf + k) < nv) {
-            if (b[k] < mn) {
-              mn = b[k];
-              jmn = 8 * hf + k;
-            }
-            if (b[k] > mx) {
-              mx = b[k];
-              jmx = 8 * hf + k;
-            }
-          }
-      }
-      if (q.out) {
-        mine[at0] = make_uint4(b[0], b[1], b[2], b[3]);
-        mine[at1] = make_uint4(b[4], b[5], b[6], b[7]);
-      }
+      for (int k = 0; k < 8; ++k)
+        b[k] = __float_as_uint(finish_score32(kMethod, kFp64 ? IPB_PRECISION_EXACT_FP64 : IPB_PRECISION_EXACT_F32,
+                                              x[k], kNeedY ? yw[k] : 0u, e.tss));
+    }
+    const uint32_t y = e.w.y0 + 8 * g + e.j;
+    const bool row_in = y < q.Ho;
+    if (q.out && row_in) {
+      float* o = q.out + (size_t)y * q.Wo + x0;
+#pragma unroll
+      for (uint32_t c = 0; c < 8; ++c)
+        if (c < nv) o[16 * c] = __uint_as_float(b[c]);
     }
     if constexpr (kExt) {
-      if (nv) {
-        const uint32_t lin = y * q.Wo + xl;
+      // scores are never negative, so their f32 bits order like the values;
+      // strict comparisons keep the first occurrence
+      uint32_t mn = 0xFFFFFFFFu, jmn = 0, mx = 0u, jmx = 0;
+#pragma unroll
+      for (uint32_t c = 0; c < 8; ++c)
+        if (c < nv) {
+          if (b[c] < mn) {
+            mn = b[c];
+            jmn = 16 * c;
+          }
+          if (b[c] > mx) {
+            mx = b[c];
+            jmx = 16 * c;
+          }
+        }
+      if (nv && row_in) {
+        const uint32_t lin = y * q.Wo + x0;
         kmin = min(kmin, ((unsigned long long)(mn | 0x80000000u) << 32) | (lin + jmn));
         kmax = max(kmax, ((unsigned long long)(mx | 0x80000000u) << 32) | (0xFFFFFFFFu - (lin + jmx)));
       }
     }
-    if (q.out) {
-      __syncwarp();
-#pragma unroll
-      for (uint32_t r = 0; r < 4; ++r) {
-        const uint32_t yr = gy0 + e.nj * r + j;
-        if (yr >= q.Ho) break;
-        const uint32_t* row = e.ytile + (e.nj * (4 * e.quad + r) + j) * kTileW;
-        float* orow = q.out + (size_t)yr * q.Wo + e.w.x0;
-#pragma unroll
-        for (uint32_t k = 0; k < 4; ++k) {
-          const uint32_t col = 32 * k + e.lane;
-          if (e.w.x0 + col < q.Wo) orow[col] = __uint_as_float(row[4 * chunk_at(col >> 2) + (col & 3u)]);
-        }
-      }
-      if (e.keep) {
-        __syncwarp();
-#pragma unroll
-        for (int k = 0; k < 4; ++k) mine[chunk_at(4 * c + k)] = ys[k];
-      }
-    }
+    __syncwarp();
   }
   if constexpr (kExt) {
     for (int o = 16; o > 0; o >>= 1) {
@@ -645,55 +625,31 @@ __device__ __forceinline__ void epilogue_m(const Epi& e, bool fp64, bool ext) {
   }
 }
 
-// The MMAs of one chunk of template rows [d0, d0 + n) for one image plane and
-// one block buffer, issued by one thread. Step t (rho = d0 + t) feeds the
-// tile's rows j = jlo .. jhi from the blocks of template rows rho - j: the
-// window of blocks grows with t until every row is fed, then moves through
-// the buffer, then shrinks.
+// The MMAs of one chunk of steps for one image plane and one block buffer,
+// issued by one thread: from step to step A moves back by one block and B down
+// by one image row.
 struct Chunk {
-  uint32_t d, a_lo, a_hi, b_lo, b_hi, row16, K, nj, d0, n;
+  uint32_t d, a_lo, a_hi, b_lo, b_hi, row16, K, steps, id;
 };
 
 template <uint32_t KSTEPS>
-__device__ __forceinline__ void issue_steps(const Chunk& c, uint32_t t0, uint32_t t1, uint32_t d, uint32_t dd,
-                                            uint32_t b, uint32_t db, uint32_t id, uint32_t did) {
-  uint32_t a = c.a_lo + (c.d0 + t0) * c.row16;
-  for (uint32_t t = t0; t < t1; ++t) {
+__device__ __forceinline__ void issue_steps(const Chunk& c) {
+  uint32_t a = c.a_lo + (c.steps - 1) * c.K, b = c.b_lo;  // 16 K bytes per block
+  for (uint32_t t = 0; t < c.steps; ++t) {
 #pragma unroll
-    for (uint32_t kk = 0; kk < KSTEPS; ++kk) mma_i8_ss(d, a + 2 * kk, c.a_hi, b + 16 * kk, c.b_hi, id, 1u);
-    a += c.row16;
-    d += dd;
-    b -= db;
-    id += did;
-  }
-}
-
-template <uint32_t KSTEPS>
-__device__ __forceinline__ void issue_chunk_k(const Chunk& c) {
-  const uint32_t m = min(c.n, c.nj), last = c.n + c.nj - 1;
-  const uint32_t one = idesc_u8u8_s32(128, 0) | (2u << 17), step = 2u << 17;  // N = 16, and 16 more
-  const uint32_t top = c.b_lo + (c.n - 1) * c.K;                              // block of template row d0
-  // growing: steps 0 .. m - 1 feed rows 0 .. t
-  issue_steps<KSTEPS>(c, 0, m, c.d, 0, top, c.K, one, step);
-  const uint32_t full = one + (m - 1) * step;
-  if (c.n >= c.nj) {
-    // all nj rows, blocks n - 1 - t down to 0
-    issue_steps<KSTEPS>(c, m, c.n, c.d, 0, top - m * c.K, c.K, full, 0);
-    issue_steps<KSTEPS>(c, c.n, last, c.d + 16, 16, c.b_lo, 0, full - step, 0u - step);
-  } else {
-    // fewer template rows than tile rows: n rows at a time, moving down the tile
-    issue_steps<KSTEPS>(c, m, c.nj, c.d + 16, 16, c.b_lo, 0, full, 0);
-    issue_steps<KSTEPS>(c, c.nj, last, c.d + 16 * (c.nj - m + 1), 16, c.b_lo, 0, full - step, 0u - step);
+    for (uint32_t kk = 0; kk < KSTEPS; ++kk) mma_i8_ss(c.d, a + 16 * kk, c.a_hi, b + 2 * kk, c.b_hi, c.id, 1u);
+    a -= c.K;
+    b += c.row16;
   }
 }
 
 __device__ __forceinline__ void issue_chunk(const Chunk& c) {
   switch (c.K / 32) {
-    case 1: issue_chunk_k<1>(c); break;
-    case 2: issue_chunk_k<2>(c); break;
-    case 3: issue_chunk_k<3>(c); break;
-    case 4: issue_chunk_k<4>(c); break;
-    default: issue_chunk_k<5>(c); break;
+    case 1: issue_steps<1>(c); break;
+    case 2: issue_steps<2>(c); break;
+    case 3: issue_steps<3>(c); break;
+    case 4: issue_steps<4>(c); break;
+    default: issue_steps<5>(c); break;
   }
 }
 
@@ -737,7 +693,7 @@ __global__ void __launch_bounds__(kThreads, 1) window_match_kernel(const __grid_
     sh->tss[0] = 0;
     mbar_init_fence();
     fence_proxy_async_smem();
-    if (P[w.pi].load_mode == 2) load_tensor(maps + w.pi, w, img, P[w.pi].tile_bytes, &sh->img_full[0]);
+    if (P[w.pi].load_mode == 2) load_tensor(maps + w.pi, !inl, w, img, P[w.pi].tile_bytes, &sh->img_full[0]);
   }
   if (P[w.pi].load_mode != 2) load_image(P[w.pi], w, img, tid, kThreads);
   load_template<MASKED>(P[w.pi], raw, L.raw_bytes, tid, kThreads);
@@ -747,8 +703,11 @@ __global__ void __launch_bounds__(kThreads, 1) window_match_kernel(const __grid_
   }
   for (uint32_t i = tid; i < kZeroRegion / 4; i += kThreads) reinterpret_cast<uint32_t*>(zero)[i] = 0u;
   __syncthreads();
-  for (uint32_t c = 0; c < min(2u, P[w.pi].nch); ++c)
-    build_chunk<MASKED>(P[w.pi], c, raw, L.raw_bytes, bslot + c * L.slot_bytes, P[w.pi].need_y, warp, kWarps, lane);
+  // chunks of the first tile that the slots hold at once
+  const uint32_t prebuilt =
+      P[w.pi].both ? 1u : min(2u, P[w.pi].nch * (MASKED && P[w.pi].need_y ? 2u : 1u));
+  for (uint32_t c = 0; c < prebuilt; ++c)
+    build_chunk(P[w.pi], c, raw, L.raw_bytes, bslot + c * L.slot_bytes, warp, kWarps, lane);
   add_tss(raw, P[w.pi].w * P[w.pi].h, &sh->tss[0], tid, kThreads);
   cp_async_wait_all();
   fence_proxy_async_smem();
@@ -764,10 +723,8 @@ __global__ void __launch_bounds__(kThreads, 1) window_match_kernel(const __grid_
     BlockState bs;
     uint32_t uses0 = 0, uses1 = 0;  // MMA uses of each block slot so far
     uint32_t claim = blockIdx.x;
-    bool pending = true;                   // a tile's image is loading, this warp has not arrived for it
-    bool tensor = P[w.pi].load_mode == 2;  // ... by a tensor copy
-    uint32_t pslot = 0;
-    int last0 = tensor ? 0 : -1, last1 = -1;  // phase of each slot's last load if by a tensor copy
+    // phase of each slot's last load if by a tensor copy (the first warp's)
+    int last0 = P[w.pi].load_mode == 2 ? 0 : -1, last1 = -1;
     for (;; ++w.ti) {
       const unsigned long long deadline = global_ns() + L.wait_ns;
       if (lt == 0) {
@@ -787,16 +744,13 @@ __global__ void __launch_bounds__(kThreads, 1) window_match_kernel(const __grid_
       const bool by_tensor = P[w.pi].load_mode == 2, need_y = P[w.pi].need_y;
       auto load = [&]() {
         const uint32_t use = w.ti / L.nbuf;  // earlier tiles in this slot
-        pending = true;
-        tensor = by_tensor;
-        pslot = slot;
         if (by_tensor && lw) return;  // the first loader warp's
         bool got = true;
         if (use) got = mbar_wait_sleep(&sh->img_empty[slot], (use - 1) & 1u, deadline);
         if (!__all_sync(0xffffffffu, got)) {
           fail = true;
         } else if (by_tensor) {
-          if (lane == 0) load_tensor(maps + w.pi, w, dst, P[w.pi].tile_bytes, &sh->img_full[slot]);
+          if (lane == 0) load_tensor(maps + w.pi, !inl, w, dst, P[w.pi].tile_bytes, &sh->img_full[slot]);
           __syncwarp();
           (slot ? last1 : last0) = (int)use;
         } else {
@@ -805,49 +759,51 @@ __global__ void __launch_bounds__(kThreads, 1) window_match_kernel(const __grid_
         }
       };
       auto publish_image = [&]() {
-        if (!by_tensor) {
-          cp_async_wait_all();
-          fence_proxy_async_smem();
-          __syncwarp();
-        }
-        if (lane == 0 && !(by_tensor && lw == 0)) mbar_arrive(&sh->img_full[slot]);
-        pending = false;
+        if (by_tensor) return;
+        cp_async_wait_all();
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sh->img_full[slot]);
       };
-      for (uint32_t m = 0; m < w.nset && !fail; ++m, ++w.it) {
+      // a wait that ran out ends the role at the next barrier, in all three
+      // warps at once
+      bool stop = false;
+      for (uint32_t m = 0; m < w.nset && !stop; ++m, ++w.it) {
         const WindowProblem q = P[w.pi + m];
-        const bool resident = bs.enter(q, m == 0 && need_y), first = w.it == 0;
+        const bool with_y = MASKED && m == 0 && need_y;
+        const bool resident = bs.enter(q, with_y), first = w.it == 0;
         uint32_t* tss = &sh->tss[w.it % (2 * kRing)];
         if (m == 0 && !first && (L.nbuf == 2 || resident)) load();
         if (!first && !resident) {
           if (lt == 0) *tss = 0;
           if (m && bar_or<kLoaders>(1, fail)) {  // the last member's blocks are built
-            fail = true;
+            stop = true;
             break;
           }
           load_template<MASKED>(q, raw, L.raw_bytes, lt, kLoaders);
           if (bar_or<kLoaders>(1, fail)) {
-            fail = true;
+            stop = true;
             break;
           }
           add_tss(raw, q.w * q.h, tss, lt, kLoaders);
         }
-        if (resident) {
-          if (lt == 0) *tss = sh->tss[(w.it - 1) % (2 * kRing)];
-          if (m == 0) publish_image();
-        }
-        for (uint32_t c = 0; c < q.nch; ++c) {
-          const uint32_t s = (bs.first + c) & 1u, uses = s ? uses1 : uses0;
-          if (s) ++uses1;
-          else ++uses0;
-          if (resident) continue;  // the MMA warp uses the chunk's slot once more
-          if (!(first && c < 2)) {
-            if (uses && !mbar_wait_sleep(&sh->b_empty[s], (uses - 1) & 1u, deadline)) fail = true;
+        if (resident && m == 0) publish_image();
+        for (uint32_t c = 0; c < q.nch * (with_y ? 2u : 1u); ++c) {
+          const uint32_t s = q.both ? 0u : (bs.first + c) & 1u;
+          // the slots' last uses first, also where the blocks stay: at most one
+          // use is outstanding, so the barriers' parities say which
+          const bool in0 = !s || q.both, in1 = s || q.both;
+          if (in0 && uses0 && !mbar_wait_sleep(&sh->b_empty[0], (uses0 - 1) & 1u, deadline)) fail = true;
+          if (in1 && uses1 && !mbar_wait_sleep(&sh->b_empty[1], (uses1 - 1) & 1u, deadline)) fail = true;
+          uses0 += in0;
+          uses1 += in1;
+          if (resident) continue;
+          if (!(first && c < prebuilt)) {
             if (bar_or<kLoaders>(1, fail)) {
-              fail = true;
+              stop = true;
               break;
             }
-            build_chunk<MASKED>(q, c, raw, L.raw_bytes, bslot + s * L.slot_bytes, m == 0 && need_y, lw, kLoadWarps,
-                                lane);
+            build_chunk(q, c, raw, L.raw_bytes, bslot + s * L.slot_bytes, lw, kLoadWarps, lane);
             fence_proxy_async_smem();
             __syncwarp();
           }
@@ -858,12 +814,13 @@ __global__ void __launch_bounds__(kThreads, 1) window_match_kernel(const __grid_
           }
         }
       }
-      if (fail) break;
+      if (stop) {
+        fail = true;
+        break;
+      }
     }
-    // no copy is in flight when the CTA leaves: a load cut short gets this
-    // warp's arrival, and the first warp waits for the tensor copies it issued
+    // no copy is in flight when the CTA leaves
     cp_async_wait_all();
-    if (pending && tensor && lw && lane == 0) mbar_arrive(&sh->img_full[pslot]);
     if (lw == 0) {
       const unsigned long long deadline = global_ns() + kDefaultWaitNs;
       if (last0 >= 0) mbar_wait_sleep(&sh->img_full[0], last0 & 1, deadline);
@@ -908,13 +865,13 @@ __global__ void __launch_bounds__(kThreads, 1) window_match_kernel(const __grid_
         }
         tc_fence_after();
         const uint32_t d = tbase + buf * accw, dy = tbase + 2 * accw;
-        const uint32_t row16 = q.pitch >> 4;
-        const uint32_t a_lo = (imga + slot * (L.plane_bytes >> 4)) | (1u << 16), a_hi = (nj * row16) | (1u << 14);
-        const uint32_t b_hi = (q.K >> 1) | (1u << 14);  // 8 K bytes between 8-row groups
+        const uint32_t row16 = q.pitch >> 4, id = idesc_u8u8_s32(128, 0) | ((accw >> 3) << 17);
+        const uint32_t a_hi = (q.K >> 1) | (1u << 14);  // 8 K bytes between 8-row groups
+        const uint32_t b_lo = (imga + slot * (L.plane_bytes >> 4)) | (1u << 16), b_hi = (8 * row16) | (1u << 14);
         if (leader) clear(d);
-        const bool resident = bs.enter(q, m == 0 && P[w.pi].need_y);
-        for (uint32_t c = 0; c < q.nch && !fail; ++c) {
-          const uint32_t s = (bs.first + c) & 1u;
+        const bool resident = bs.enter(q, with_y);
+        for (uint32_t cc = 0; cc < q.nch * (with_y ? 2u : 1u) && !fail; ++cc) {
+          const uint32_t s = q.both ? 0u : (bs.first + cc) & 1u, c = cc < q.nch ? cc : cc - q.nch;
           if (!resident) {
             const uint32_t builds = s ? builds1++ : builds0++;
             if (!__all_sync(0xffffffffu, mbar_wait(&sh->b_full[s], builds & 1u, deadline))) {
@@ -923,35 +880,37 @@ __global__ void __launch_bounds__(kThreads, 1) window_match_kernel(const __grid_
             }
             tc_fence_after();
           }
-          const uint32_t d0 = c * q.crows, n = min(q.crows, q.h - d0);
-          const uint32_t b_lo = (ba + s * (L.slot_bytes >> 4)) | (8u << 16);
-          if (leader) issue_chunk(Chunk{d, a_lo, a_hi, b_lo, b_hi, row16, q.K, nj, d0, n});
-          __syncwarp();
-          if constexpr (MASKED) {
-            if (with_y) {
-              if (!planes_ready) {
-                got = mbar_wait(&sh->planes_full, w.ti & 1u, deadline);
-                if (ytiles) got = got && mbar_wait(&sh->yacc_empty, (ytiles - 1) & 1u, deadline);
-                if (!__all_sync(0xffffffffu, got)) {
-                  fail = true;
-                  break;
-                }
-                tc_fence_after();
-                planes_ready = true;
-                ++ytiles;
-                if (leader) {
-                  clear(dy);
-                  clear(dy + accw);
-                }
+          const uint32_t r0 = c * q.csteps, steps = min(q.csteps, q.h + 7 - r0);
+          const uint32_t a_lo = (ba + s * (L.slot_bytes >> 4)) | (8u << 16);
+          if (!MASKED || cc < q.nch) {
+            if (leader) issue_chunk(Chunk{d, a_lo, a_hi, b_lo + r0 * row16, b_hi, row16, q.K, steps, id});
+          } else {
+            if (!planes_ready) {
+              got = mbar_wait(&sh->planes_full, w.ti & 1u, deadline);
+              if (ytiles) got = got && mbar_wait(&sh->yacc_empty, (ytiles - 1) & 1u, deadline);
+              if (!__all_sync(0xffffffffu, got)) {
+                fail = true;
+                break;
               }
-              if (leader)
-                for (uint32_t p = 0; p < 2; ++p)
-                  issue_chunk(Chunk{dy + p * accw, (pla + p * (L.plane_bytes >> 4)) | (1u << 16), a_hi,
-                                    b_lo + q.crows * q.K, b_hi, row16, q.K, nj, d0, n});
-              __syncwarp();
+              tc_fence_after();
+              planes_ready = true;
+              ++ytiles;
+              if (leader) {
+                clear(dy);
+                clear(dy + accw);
+              }
             }
+            if (leader)
+              for (uint32_t p = 0; p < 2; ++p)
+                issue_chunk(Chunk{dy + p * accw, a_lo, a_hi,
+                                  ((pla + p * (L.plane_bytes >> 4)) | (1u << 16)) + r0 * row16, b_hi, row16, q.K, steps,
+                                  id});
           }
-          if (leader) mma_commit(&sh->b_empty[s]);
+          __syncwarp();
+          if (leader) {
+            if (!s || q.both) mma_commit(&sh->b_empty[0]);
+            if (s || q.both) mma_commit(&sh->b_empty[1]);
+          }
           __syncwarp();
         }
         if (fail) break;
@@ -977,28 +936,27 @@ __global__ void __launch_bounds__(kThreads, 1) window_match_kernel(const __grid_
     if (!mbar_wait(&sh->drain, 0, global_ns() + kDefaultWaitNs) && lane == 0) atomicMax(L.err, L.tag);
   } else {
     // ---- workers: window sums (unmasked) or planes of I^2 (masked) of a tile
-    // beside its MMAs, then the epilogue of each of its set's members. A
-    // quadrant's four warps share the rows of its lane groups: each forms one
-    // group's window sums, then scores a quarter of every group's rows.
+    // beside its MMAs, then the epilogue of each of its set's members. The four
+    // warps of a quarter (one per tensor-memory lane quadrant) share a quarter
+    // of the tile's rows: each forms the window sums of a quarter of those,
+    // then scores two rows of every group of eight (of a 16-row tile, whose two
+    // groups span quarters, all warps wait for one another).
     const uint32_t quad = warp & 3, sub = warp >> 2;
-    const uint32_t j0 = sub * nj / 4, j1 = (sub + 1) * nj / 4;
+    const uint32_t g0 = sub * 2 * nj / 4, g1 = (sub + 1) * 2 * nj / 4;
+    const bool together = MASKED || nj == 1;
+    uint32_t tss = 0, tss_of = 0xFFFFFFFFu;  // sum (T m)^2 and the problem it is of
     for (;; ++w.ti) {
       const unsigned long long deadline = global_ns() + L.wait_ns;
       const bool more = next_tile<false>(w, L, P, sh, deadline);
       fail = __any_sync(0xffffffffu, fail || !w.ok);
-      if constexpr (MASKED) {
-        // the planes replace the last tile's window sums
-        if (bar_or<kWorkWarps * 32>(6, fail)) {
-          fail = true;
-          break;
-        }
-      }
       const uint32_t slot = L.nbuf == 2 ? (w.ti & 1u) : 0u;
       const bool need_y = P[w.pi].need_y;
       if (more && !fail) {
+        // waited for also where nothing is read, so that no warp arrives for a
+        // tile while another still reads the last one
+        const bool got = mbar_wait_sleep(&sh->img_full[slot], (w.ti / L.nbuf) & 1u, deadline);
+        if (!__all_sync(0xffffffffu, got)) fail = true;
         if (need_y) {
-          const bool got = mbar_wait_sleep(&sh->img_full[slot], (w.ti / L.nbuf) & 1u, deadline);
-          if (!__all_sync(0xffffffffu, got)) fail = true;
           const WindowProblem& q = P[w.pi];
           const uint8_t* src = img + slot * L.plane_bytes;
           if constexpr (MASKED) {
@@ -1015,7 +973,7 @@ __global__ void __launch_bounds__(kThreads, 1) window_match_kernel(const __grid_
               }
             fence_proxy_async_smem();
           } else if (!fail) {
-            window_sums_dispatch(src, q.pitch, q.w, q.h, nj * (4 * quad + sub), nj, lane, ytile);
+            window_sums_dispatch(src, q.pitch, q.w, q.h, nj * (4 * sub + quad), nj, lane, ytile);
           }
         }
         __syncwarp();
@@ -1024,7 +982,7 @@ __global__ void __launch_bounds__(kThreads, 1) window_match_kernel(const __grid_
           if constexpr (MASKED) mbar_arrive(&sh->planes_full);
         }
       }
-      if (bar_or<128>(2 + quad, fail)) {
+      if (together ? bar_or<kWorkWarps * 32>(6, fail) : bar_or<128>(2 + sub, fail)) {
         fail = true;
         break;
       }
@@ -1038,14 +996,19 @@ __global__ void __launch_bounds__(kThreads, 1) window_match_kernel(const __grid_
           break;
         }
         tc_fence_after();
-        const uint32_t tss = *reinterpret_cast<volatile uint32_t*>(&sh->tss[w.it % (2 * kRing)]);
+        // a template that follows itself may have stayed in its slots; its sum
+        // is then not handed over again
+        if (tss_of == 0xFFFFFFFFu || P[tss_of].tpl != q.tpl || P[tss_of].mask != q.mask || P[tss_of].w != q.w ||
+            P[tss_of].h != q.h)
+          tss = *reinterpret_cast<volatile uint32_t*>(&sh->tss[w.it % (2 * kRing)]);
+        tss_of = w.pi + m;
         const double td = u32_to_double(tss);
         const uint32_t acc = tmem_addr(tbase, 32 * quad, 0);
-        const Epi e{q, w, nj, acc + buf * accw, accw, quad, lane, j0, j1, tss, td, -4503599627370496.0 * td, ytile,
-                    need_y && m + 1 < w.nset};
+        const Epi e{q, w, acc + buf * accw, 2 * quad + ((uint32_t)lane >> 4), (uint32_t)lane & 15u, (uint32_t)lane, g0, g1,
+                    tss, td, -4503599627370496.0 * td, ytile};
         if constexpr (MASKED) {
           if (need_y && m == 0) {
-            gather_sums(e, acc + 2 * accw);
+            gather_sums(e, acc + 2 * accw, acc + 3 * accw);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&sh->yacc_empty);
@@ -1062,8 +1025,9 @@ __global__ void __launch_bounds__(kThreads, 1) window_match_kernel(const __grid_
         __syncwarp();
         if (lane == 0) mbar_arrive(&sh->acc_empty[buf]);
       }
-      // the quadrant's rows hold the next tile's window sums from here on
-      if (bar_or<128>(2 + quad, fail)) {
+      // the quarter's rows hold the next tile's window sums from here on (all
+      // rows, its planes of I^2)
+      if (together ? bar_or<kWorkWarps * 32>(6, fail) : bar_or<128>(2 + sub, fail)) {
         fail = true;
         break;
       }
@@ -1117,7 +1081,11 @@ bool window_supported(const MatchArgs& a) {
   if (a.precision == IPB_PRECISION_REFERENCE_F32 || (a.mask && !a.mask_binary)) return false;
   if (a.w < 1 || a.h < 1 || a.w > kMaxSide || a.h > kMaxSide || a.w > a.W || a.h > a.H) return false;
   // tile indices are 32-bit whatever the tile height
-  return (uint64_t)((a.W - a.w) / kTileW + 1) * ((a.H - a.h) / 16 + 1) < 0xFFFF0000ull;
+  if ((uint64_t)((a.W - a.w) / kTileW + 1) * ((a.H - a.h) / 16 + 1) >= 0xFFFF0000ull) return false;
+  // the largest masked templates leave too little shared memory beside the
+  // image and its planes for tiles of 64 rows: the Hankel-row kernel's
+  WindowPlan pl;
+  return !a.mask || window_plan_for(a.w, a.h, true, 4, 1, pl);
 }
 
 bool window_plan_for(uint32_t wmax, uint32_t hmax, bool masked, uint32_t nj, uint32_t nbuf, WindowPlan& pl) {
@@ -1136,10 +1104,11 @@ bool window_plan_for(uint32_t wmax, uint32_t hmax, bool masked, uint32_t nj, uin
   const uint32_t raw = pl.raw_bytes * (masked ? 2u : 1u);
   if (pl.b_off + raw >= kSmemMax) return false;
   pl.slot_bytes = (kSmemMax - pl.b_off - raw) / 2 & ~127u;
-  const uint32_t block = 16 * K * (masked ? 2u : 1u);
-  // a template needs no more than a slot of its own size
-  pl.slot_bytes = std::min(pl.slot_bytes, (uint32_t)align_up((size_t)hmax * block, 128));
-  if (pl.slot_bytes < 8 * block && pl.slot_bytes < hmax * block) return false;
+  const uint32_t block = 16 * K;
+  // a template needs no more than a slot of its own size; chunks of fewer than
+  // eight steps would build more than they use
+  pl.slot_bytes = std::min(pl.slot_bytes, (uint32_t)align_up((size_t)(hmax + 14) * block, 128));
+  if (pl.slot_bytes < 15 * block) return false;
   pl.raw_off = pl.b_off + 2 * pl.slot_bytes;
   pl.smem = std::max(kMinSmem, pl.raw_off + raw);
   return pl.smem <= kSmemMax;
@@ -1149,7 +1118,7 @@ bool window_plan_for(uint32_t wmax, uint32_t hmax, bool masked, uint32_t nj, uin
 // them (its blocks then stay from tile to tile), else one.
 bool window_plan_best(uint32_t wmax, uint32_t hmax, bool masked, uint32_t nj, WindowPlan& pl) {
   if (!masked && window_plan_for(wmax, hmax, masked, nj, 2, pl) &&
-      2 * (pl.slot_bytes / (16 * k_of(wmax))) >= hmax)
+      2 * pl.slot_bytes / (16 * k_of(wmax)) >= hmax + 14)
     return true;
   return window_plan_for(wmax, hmax, masked, nj, 1, pl);
 }
@@ -1170,9 +1139,13 @@ WindowProblem window_problem(const MatchArgs& a, const WindowPlan& pl, unsigned 
   q.tiles_x = (q.Wo + kTileW - 1) / kTileW;
   q.K = k_of(a.w);
   q.pitch = pitch_of(a.w);
-  const uint32_t fit = pl.slot_bytes / (16 * q.K * (a.mask ? 2u : 1u));  // template rows per slot
-  q.nch = (a.h + fit - 1) / fit;
-  q.crows = (a.h + q.nch - 1) / q.nch;
+  // steps 0 .. h + 6 in chunks of csteps, csteps + 7 blocks each: one chunk in
+  // a slot, one over both slots (it then stays, but the next template's blocks
+  // wait for its last MMA), or as many as it takes
+  const uint32_t block = 16 * q.K, fit = pl.slot_bytes / block, steps = a.h + 7;
+  q.both = steps + 7 > fit && steps + 7 <= 2 * pl.slot_bytes / block;
+  q.nch = q.both ? 1u : (steps + fit - 8) / (fit - 7);
+  q.csteps = (steps + q.nch - 1) / q.nch;
   const uintptr_t ia = reinterpret_cast<uintptr_t>(a.img);
   q.load_mode = ((ia & 3u) == 0 && (a.W & 3u) == 0) ? 1 : 0;
   const uint32_t rows = 16 * pl.nj + a.h - 1;
@@ -1284,8 +1257,7 @@ uint32_t window_tile_nj(const MatchArgs& a, uint32_t n, uint32_t set) {
   uint32_t nj_best = 8;
   for (uint32_t nj : {8u, 4u, 2u, 1u}) {
     const uint64_t tiles = (uint64_t)((Wo + kTileW - 1) / kTileW) * ((Ho + 16 * nj - 1) / (16 * nj)) * nsets;
-    const double full = std::max(32.0 + 4.0 * nj, 8.0 * nj), part = 32.0 + 2.0 * nj;
-    const double steps = (a.h >= nj ? a.h - nj + 1 : 1) * full + 2.0 * (nj - 1) * part;
+    const double steps = (a.h + 7.0) * std::max(32.0 + 4.0 * nj, 8.0 * nj);
     const double corr = (double)((n + nsets - 1) / nsets) + (a.mask ? 2.0 : 0.0);
     const double unit = corr * (k_of(a.w) / 32) * steps + 1000.0 * nj;
     const double cost = (double)((tiles + sms - 1) / sms) * unit + 6000.0;

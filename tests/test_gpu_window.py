@@ -1,4 +1,4 @@
-"""The window kernel (staged image tiles read in place as the A operand)
+"""The window kernel (staged image tiles read in place as an MMA operand)
 against the oracle, bit for bit.
 
 Shapes sit at the kernel's edges: template widths where the K of the MMAs or
@@ -81,11 +81,13 @@ def test_window_kernel_unaligned_buffers_and_sets(offset, tmp_path, monkeypatch)
         return view
 
     items, dev_items = [], []
-    for W, H, w, h in ((512, 300, 40, 24), (301, 260, 64, 70), (640, 129, 8, 100)):
+    for W, H, w, h in ((512, 300, 40, 24), (301, 260, 64, 64), (640, 129, 8, 100), (700, 500, 64, 40),
+                       (400, 300, 128, 128)):
         image, t0, mask = scene(W, H, w, h)
         t1 = t0[::-1].copy()
         di, d0, d1, dm = dev(image), dev(t0), dev(t1), dev(mask)
-        for t, d, method in ((t0, d0, 2), (t0, d0, 3), (t1, d1, 0), (t1, d1, 1), (t0, d0, 1)):
+        # sets of four: one template three times, then another
+        for t, d, method in ((t0, d0, 2), (t0, d0, 3), (t1, d1, 0), (t0, d0, 1)):
             items += [(image, t, method, None), (image, t, method, mask)]
             dev_items += [(di, d, method), (di, d, method, dm)]
     batch = device.Batch(dev_items)
@@ -102,4 +104,39 @@ def test_window_kernel_unaligned_buffers_and_sets(offset, tmp_path, monkeypatch)
             mx, mn, mxl, mnl = O.find_extremes(exp)
             assert (e.max_value, e.min_value, e.max_value_location, e.min_value_location) == \
                 (float(mx), float(mn), mxl, mnl), k
+    plan.close()
+
+
+@pytest.mark.parametrize("tune", [False, True])
+def test_window_kernel_mixed_group(tune, tmp_path, monkeypatch):
+    # more problems in a launch than its parameters hold, of unequal sizes: a
+    # CTA passes from templates of one chunk to ones over both block slots and
+    # in many chunks, from sets that need window sums to sets that do not, and
+    # takes several tiles of one template in a row, staged by tensor copies
+    # (rows on 16-byte boundaries) and without
+    import torch
+
+    from imageproc_b200 import _lib, device
+    monkeypatch.setenv("IPB_AUTOTUNE", "1" if tune else "0")
+    monkeypatch.setenv("IPB_TUNING_FILE", "")
+    _lib.lib().ipb_batch_tuning_reset()
+    sizes = [(2720, 2704, 25, 6, 2), (2720, 1500, 9, 4, 3), (1601, 700, 31, 17, 0), (640, 400, 18, 120, 1),
+             (333, 444, 12, 97, 2), (512, 512, 29, 61, 3), (410, 300, 17, 1, 2), (800, 600, 32, 45, 1),
+             (257, 258, 8, 109, 0), (1200, 900, 24, 30, 2), (448, 300, 30, 104, 3)]
+    items, dev_items = [], []
+    for W, H, w, h, method in sizes:
+        image, t, _ = scene(W, H, w, h)
+        items.append((image, t, method))
+        dev_items.append((torch.from_numpy(image).cuda(), torch.from_numpy(t).cuda(), method))
+    batch = device.Batch(dev_items)
+    plan = device.BatchPlan(batch)
+    exp = [O.match_exact(image, t, method, precision=0) for image, t, method in items]
+    for _ in range(3):
+        for o in batch.outs:
+            o.fill_(-1.0)
+        plan.launch()
+        torch.cuda.synchronize()
+        for k, (want, out) in enumerate(zip(exp, batch.outs)):
+            bad = np.argwhere(bits(out.cpu().numpy()) != bits(want))
+            assert bad.size == 0, (sizes[k], bad[:3])
     plan.close()
