@@ -80,15 +80,10 @@ constexpr uint32_t kWarps = kLoadWarp + kLoadWarps, kThreads = kWarps * 32, kLoa
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kRing = 8;  // tile indices in flight: roles are at most four tiles apart
 constexpr uint32_t kHeader = 1024;
-// the zero operands of the clearing MMA: 128 rows 16 bytes apart, 32 bytes each
-constexpr uint32_t kZeroBytes = 16 * 127 + 32;
-constexpr uint32_t kZeroRegion = 2176;
-constexpr uint32_t kFixed = kHeader + kZeroRegion;
+constexpr uint32_t kFixed = kHeader;
 constexpr uint32_t kSmemMax = 227 * 1024;
 constexpr uint32_t kMinSmem = 120 * 1024;  // one CTA per SM: two never wait on each other's tensor memory
 constexpr uint32_t kMaxSide = 128;         // template width and height
-
-static_assert(kZeroBytes <= kZeroRegion, "zero operands");
 
 __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src, uint32_t src_bytes) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
@@ -257,26 +252,44 @@ __device__ __forceinline__ void load_tensor(const CUtensorMap* map, bool global,
       : "memory");
 }
 
-// The template (plane 0: T or T m) and, masked, the mask (plane 1) as they lie
-// in memory, by words, zero past the end.
+// Bytes [x, x + 4) of a w-byte row that starts at p, zero past its end, read
+// as aligned words where those lie inside [p0, end).
+__device__ __forceinline__ uint32_t row_word(const uint8_t* p, uint32_t x, uint32_t w, const uint8_t* p0,
+                                             const uint8_t* end) {
+  if (x >= w) return 0u;
+  const uint8_t* g = p + x;
+  const uint32_t off = (uint32_t)(reinterpret_cast<uintptr_t>(g) & 3u), n = min(4u, w - x);
+  const uint8_t* a = g - off;
+  if (a >= p0 && a + 8 <= end) {
+    const uint32_t* a4 = reinterpret_cast<const uint32_t*>(a);
+    const uint32_t v = __byte_perm(__ldg(a4), __ldg(a4 + 1), 0x3210u + off * 0x1111u);
+    return n == 4 ? v : v & ((1u << (8 * n)) - 1u);
+  }
+  uint32_t v = 0;
+#pragma unroll
+  for (uint32_t k = 0; k < 4; ++k)
+    if (k < n) v |= (uint32_t)__ldg(g + k) << (8 * k);
+  return v;
+}
+
+// The template (T or T m) and, masked, the mask behind it, as rows of K bytes,
+// zero past the row's w (at least 15 zeros, which are also the zeros ahead of
+// the next row; sixteen more lie ahead of the first).
 template <bool MASKED>
 __device__ __forceinline__ void load_template(const WindowProblem& q, uint8_t* raw, uint32_t raw_bytes, uint32_t t,
                                               uint32_t nt) {
-  const uint32_t n = q.w * q.h, words = (n + 3) / 4;
-  const bool aligned = ((reinterpret_cast<uintptr_t>(q.tpl) | (MASKED ? reinterpret_cast<uintptr_t>(q.mask) : 0)) & 3u) == 0;
-  auto word = [&](const uint8_t* p, uint32_t i) {
-    if (aligned && 4 * i + 4 <= n) return __ldg(reinterpret_cast<const uint32_t*>(p) + i);
-    uint32_t v = 0;
-#pragma unroll
-    for (uint32_t k = 0; k < 4; ++k)
-      if (4 * i + k < n) v |= (uint32_t)__ldg(p + 4 * i + k) << (8 * k);
-    return v;
-  };
-#pragma unroll 8
-  for (uint32_t i = t; i < words; i += nt) {
-    uint32_t v = word(q.tpl, i);
+  const uint32_t words = q.K / 4, n = q.h * words;
+  const uint8_t *tend = q.tpl + q.w * q.h, *mend = MASKED ? q.mask + q.w * q.h : nullptr;
+  if (t < 4) {
+    reinterpret_cast<uint32_t*>(raw - 16)[t] = 0u;
+    if constexpr (MASKED) reinterpret_cast<uint32_t*>(raw + raw_bytes - 16)[t] = 0u;
+  }
+#pragma unroll 4
+  for (uint32_t i = t; i < n; i += nt) {
+    const uint32_t r = i / words, x = (i - r * words) * 4;
+    uint32_t v = row_word(q.tpl + r * q.w, x, q.w, q.tpl, tend);
     if constexpr (MASKED) {
-      const uint32_t m = word(q.mask, i);
+      const uint32_t m = row_word(q.mask + r * q.w, x, q.w, q.mask, mend);
       v &= m * 255u;  // bytes of m are 0 or 1
       reinterpret_cast<uint32_t*>(raw + raw_bytes)[i] = m;
     }
@@ -286,9 +299,9 @@ __device__ __forceinline__ void load_template(const WindowProblem& q, uint8_t* r
 
 // Adds sum T^2 of the words in shared memory (u32: at most 16384 template
 // pixels) to *tss, by `nt` threads in whole warps.
-__device__ __forceinline__ void add_tss(const uint8_t* raw, uint32_t pixels, uint32_t* tss, uint32_t t, uint32_t nt) {
+__device__ __forceinline__ void add_tss(const uint8_t* raw, uint32_t words, uint32_t* tss, uint32_t t, uint32_t nt) {
   uint32_t t2 = 0;
-  for (uint32_t i = t; i < (pixels + 3) / 4; i += nt) {
+  for (uint32_t i = t; i < words; i += nt) {
     const uint32_t v = reinterpret_cast<const uint32_t*>(raw)[i];
     t2 = __dp4a(v, v, t2);
   }
@@ -298,55 +311,41 @@ __device__ __forceinline__ void add_tss(const uint8_t* raw, uint32_t pixels, uin
 
 // The 16-shift blocks of n consecutive template rows in decreasing order from
 // row `top` (rows outside the template are zero): block b holds rows s = 0..15
-// of K bytes, byte k = T[top - b][k - s] (0 outside the row), in the canonical
-// no-swizzle K-major layout (s / 8) 8K + (k / 16) 128 + (s % 8) 16. A warp
-// writes four core matrices (512 bytes) of a row at once; the K / 32 such
-// groups of all rows are shared out over `nw` warps group by group, so that a
-// lane mostly keeps its shift, its chunk and the bytes of it that lie in the
-// row while it goes down the rows.
-__device__ __forceinline__ void build_blocks(uint32_t K, uint32_t w, uint32_t h, uint32_t top, uint32_t n,
-                                             const uint8_t* raw, uint8_t* dst, uint32_t iw, uint32_t nw,
-                                             uint32_t lane) {
-  const uint32_t cpr = K / 16, items = (K / 32) * n;
-  uint32_t item = iw * items / nw;
-  const uint32_t end = (iw + 1) * items / nw;
-  while (item < end) {
-    const uint32_t grp = item / n, b_end = min(n, end - grp * n);
-    const uint32_t m = 4 * grp + (lane >> 3);
-    const uint32_t hi = m >= cpr ? 1u : 0u, ch = m - hi * cpr, sft = 8 * hi + (lane & 7u);
-    uint32_t mask[4];
+// of K bytes, byte k = T[top - b][k - s] (0 outside the row), in the no-swizzle
+// K-major layout (s / 8) (8K + 16) + (k / 16) 128 + (s % 8) 16. A thread takes
+// one 16-byte chunk and eight shifts of a row: a window of 24 bytes, from
+// which every shift is a fixed byte selection. The 16 bytes of padding per
+// eight rows spread the stores of four blocks and both halves over all banks.
+// (A lane per shift read five words per 16-byte unit: 3000 cycles for the 64
+// rows of a 64 x 64 template by 20 warps, this 700.)
+__device__ __forceinline__ void build_blocks(uint32_t K, uint32_t h, uint32_t top, uint32_t n, const uint8_t* raw,
+                                             uint8_t* dst, uint32_t t, uint32_t nt) {
+  const uint32_t cpr = K / 16, items = 8 * cpr * ((n + 3) / 4);
+  for (uint32_t i = t; i < items; i += nt) {
+    const uint32_t hi = i & 1u, rest = i >> 3, quad = rest / cpr, ch = rest - quad * cpr;
+    const uint32_t b = 4 * quad + ((i >> 1) & 3u), d = top - b;  // wraps below row 0
+    if (b >= n) continue;
+    uint32_t w[6] = {0u, 0u, 0u, 0u, 0u, 0u};
+    if (d < h) {
+      const uint2* src = reinterpret_cast<const uint2*>(raw + (int)(d * K + 16 * ch) - 8 * (int)hi - 8);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      mask[i] = 0;
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-        if (16 * ch + 4 * i + k - sft < w) mask[i] |= 0xFFu << (8 * k);  // wraps for the bytes ahead of the row
-    }
-    uint8_t* out = dst + m * 128 + (lane & 7u) * 16;
-    const uint32_t first = 16 + 16 * ch - sft;  // sixteen bytes of slack lie ahead of the template
-    // four rows' reads ahead of their stores
-    for (uint32_t b0 = item - grp * n; b0 < b_end; b0 += 4) {
-      uint32_t wd[4][5], sel[4], ok[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const uint32_t d = top - (b0 + i);  // wraps below row 0
-        ok[i] = d < h ? 0xFFFFFFFFu : 0u;
-        const uint32_t at = first + (d < h ? d : 0u) * w;
-        const uint32_t* a4 = reinterpret_cast<const uint32_t*>(raw - 16 + (at & ~3u));
-        sel[i] = 0x3210u + (at & 3u) * 0x1111u;
-#pragma unroll
-        for (int k = 0; k < 5; ++k) wd[i][k] = a4[k];
+      for (int k = 0; k < 3; ++k) {
+        const uint2 v = src[k];
+        w[2 * k] = v.x;
+        w[2 * k + 1] = v.y;
       }
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        if (b0 + i < b_end)
-          *reinterpret_cast<uint4*>(out + (b0 + i) * 16 * K) =
-              make_uint4(__byte_perm(wd[i][0], wd[i][1], sel[i]) & mask[0] & ok[i],
-                         __byte_perm(wd[i][1], wd[i][2], sel[i]) & mask[1] & ok[i],
-                         __byte_perm(wd[i][2], wd[i][3], sel[i]) & mask[2] & ok[i],
-                         __byte_perm(wd[i][3], wd[i][4], sel[i]) & mask[3] & ok[i]);
     }
-    item = grp * n + b_end;
+    uint4* out = reinterpret_cast<uint4*>(dst + b * (16 * K + 32) + hi * (8 * K + 16) + ch * 128);
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {
+      const int o = 8 - s, f = o >> 2;  // first byte of the shift's sixteen in the window, its word
+      const uint32_t sel = 0x3210u + (uint32_t)(o & 3) * 0x1111u;
+      if ((o & 3) == 0)
+        out[s] = make_uint4(w[f], w[f + 1], w[f + 2], w[f + 3]);
+      else
+        out[s] = make_uint4(__byte_perm(w[f], w[f + 1], sel), __byte_perm(w[f + 1], w[f + 2], sel),
+                            __byte_perm(w[f + 2], w[f + 3], sel), __byte_perm(w[f + 3], w[f + 4], sel));
+    }
   }
 }
 
@@ -354,11 +353,10 @@ __device__ __forceinline__ void build_blocks(uint32_t K, uint32_t w, uint32_t h,
 // its steps [r0, r1); the template's chunks first, then (masked sets that need
 // window sums) the mask's.
 __device__ __forceinline__ void build_chunk(const WindowProblem& q, uint32_t cc, const uint8_t* raw,
-                                            uint32_t raw_bytes, uint8_t* slot, uint32_t iw, uint32_t nw,
-                                            uint32_t lane) {
+                                            uint32_t raw_bytes, uint8_t* slot, uint32_t t, uint32_t nt) {
   const uint32_t c = cc < q.nch ? cc : cc - q.nch;
   const uint32_t r0 = c * q.csteps, r1 = min(r0 + q.csteps, q.h + 7);
-  build_blocks(q.K, q.w, q.h, r1 - 1, r1 - r0 + 7, cc < q.nch ? raw : raw + raw_bytes, slot, iw, nw, lane);
+  build_blocks(q.K, q.h, r1 - 1, r1 - r0 + 7, cc < q.nch ? raw : raw + raw_bytes, slot, t, nt);
 }
 
 __device__ __forceinline__ void add_squares(uint2 v, uint32_t (&a)[8]) {
@@ -630,15 +628,20 @@ __device__ __forceinline__ void epilogue_m(const Epi& e, bool fp64, bool ext) {
 // by one image row.
 struct Chunk {
   uint32_t d, a_lo, a_hi, b_lo, b_hi, row16, K, steps, id;
+  bool clear;  // the accumulator's first chunk: its first MMA overwrites
 };
 
 template <uint32_t KSTEPS>
 __device__ __forceinline__ void issue_steps(const Chunk& c) {
-  uint32_t a = c.a_lo + (c.steps - 1) * c.K, b = c.b_lo;  // 16 K bytes per block
+  const uint32_t blk = c.K + 2;  // 16 K + 32 bytes per block
+  uint32_t a = c.a_lo + (c.steps - 1) * blk, b = c.b_lo, acc = c.clear ? 0u : 1u;
   for (uint32_t t = 0; t < c.steps; ++t) {
 #pragma unroll
-    for (uint32_t kk = 0; kk < KSTEPS; ++kk) mma_i8_ss(c.d, a + 16 * kk, c.a_hi, b + 2 * kk, c.b_hi, c.id, 1u);
-    a -= c.K;
+    for (uint32_t kk = 0; kk < KSTEPS; ++kk) {
+      mma_i8_ss(c.d, a + 16 * kk, c.a_hi, b + 2 * kk, c.b_hi, c.id, acc);
+      acc = 1u;
+    }
+    a -= blk;
     b += c.row16;
   }
 }
@@ -657,14 +660,13 @@ template <bool MASKED>
 __global__ void __launch_bounds__(kThreads, 1) window_match_kernel(const __grid_constant__ WindowLaunch L) {
   extern __shared__ __align__(1024) uint8_t smem[];
   Shared* sh = reinterpret_cast<Shared*>(smem);
-  uint8_t* zero = smem + kHeader;
   // window sums of the tile; masked, in the place of its planes of I^2 (low
   // bytes, high bytes), which no MMA reads any more by then
   uint32_t* ytile = reinterpret_cast<uint32_t*>(smem + kFixed);
   uint8_t* planes = smem + kFixed;
   uint8_t* img = smem + L.img_off;
   uint8_t* bslot = smem + L.b_off;
-  uint8_t* raw = smem + L.raw_off + 16;  // the template as it lies in memory
+  uint8_t* raw = smem + L.raw_off + 16;  // the template's rows
   const bool inl = L.nprobs <= kInlineProblems;
   const WindowProblem* P = inl ? L.inl : L.probs;
   const CUtensorMap* maps = inl ? L.inl_maps : L.maps;
@@ -701,14 +703,13 @@ __global__ void __launch_bounds__(kThreads, 1) window_match_kernel(const __grid_
     tmem_alloc(&sh->tmem, kTmemCols);
     tmem_relinquish();
   }
-  for (uint32_t i = tid; i < kZeroRegion / 4; i += kThreads) reinterpret_cast<uint32_t*>(zero)[i] = 0u;
   __syncthreads();
   // chunks of the first tile that the slots hold at once
   const uint32_t prebuilt =
       P[w.pi].both ? 1u : min(2u, P[w.pi].nch * (MASKED && P[w.pi].need_y ? 2u : 1u));
   for (uint32_t c = 0; c < prebuilt; ++c)
-    build_chunk(P[w.pi], c, raw, L.raw_bytes, bslot + c * L.slot_bytes, warp, kWarps, lane);
-  add_tss(raw, P[w.pi].w * P[w.pi].h, &sh->tss[0], tid, kThreads);
+    build_chunk(P[w.pi], c, raw, L.raw_bytes, bslot + c * L.slot_bytes, tid, kThreads);
+  add_tss(raw, P[w.pi].h * (P[w.pi].K / 4), &sh->tss[0], tid, kThreads);
   cp_async_wait_all();
   fence_proxy_async_smem();
   tc_fence_before();
@@ -785,7 +786,7 @@ __global__ void __launch_bounds__(kThreads, 1) window_match_kernel(const __grid_
             stop = true;
             break;
           }
-          add_tss(raw, q.w * q.h, tss, lt, kLoaders);
+          add_tss(raw, q.h * (q.K / 4), tss, lt, kLoaders);
         }
         if (resident && m == 0) publish_image();
         for (uint32_t c = 0; c < q.nch * (with_y ? 2u : 1u); ++c) {
@@ -803,7 +804,7 @@ __global__ void __launch_bounds__(kThreads, 1) window_match_kernel(const __grid_
               stop = true;
               break;
             }
-            build_chunk(q, c, raw, L.raw_bytes, bslot + s * L.slot_bytes, lw, kLoadWarps, lane);
+            build_chunk(q, c, raw, L.raw_bytes, bslot + s * L.slot_bytes, lt, kLoaders);
             fence_proxy_async_smem();
             __syncwarp();
           }
@@ -831,12 +832,7 @@ __global__ void __launch_bounds__(kThreads, 1) window_match_kernel(const __grid_
     BlockState bs;
     uint32_t builds0 = 0, builds1 = 0, ytiles = 0;
     const bool leader = elect_one();
-    const uint32_t z = smem_u32(zero) >> 4, imga = smem_u32(img) >> 4, pla = smem_u32(planes) >> 4,
-                   ba = smem_u32(bslot) >> 4;
-    auto clear = [&](uint32_t d) {
-      const uint32_t id = idesc_u8u8_s32(128, 0) | ((accw >> 3) << 17);
-      mma_i8_ss(d, z | (1u << 16), 8u | (1u << 14), z | (1u << 16), 8u | (1u << 14), id, 0u);
-    };
+    const uint32_t imga = smem_u32(img) >> 4, pla = smem_u32(planes) >> 4, ba = smem_u32(bslot) >> 4;
     // test hook: a wait on the drain barrier, which nothing arrives at before the end
     if (L.stall && !mbar_wait(&sh->drain, 0, global_ns() + L.wait_ns)) fail = true;
     fail = __any_sync(0xffffffffu, fail);
@@ -866,9 +862,8 @@ __global__ void __launch_bounds__(kThreads, 1) window_match_kernel(const __grid_
         tc_fence_after();
         const uint32_t d = tbase + buf * accw, dy = tbase + 2 * accw;
         const uint32_t row16 = q.pitch >> 4, id = idesc_u8u8_s32(128, 0) | ((accw >> 3) << 17);
-        const uint32_t a_hi = (q.K >> 1) | (1u << 14);  // 8 K bytes between 8-row groups
+        const uint32_t a_hi = ((q.K >> 1) + 1u) | (1u << 14);  // 8 K + 16 bytes between 8-row groups
         const uint32_t b_lo = (imga + slot * (L.plane_bytes >> 4)) | (1u << 16), b_hi = (8 * row16) | (1u << 14);
-        if (leader) clear(d);
         const bool resident = bs.enter(q, with_y);
         for (uint32_t cc = 0; cc < q.nch * (with_y ? 2u : 1u) && !fail; ++cc) {
           const uint32_t s = q.both ? 0u : (bs.first + cc) & 1u, c = cc < q.nch ? cc : cc - q.nch;
@@ -883,7 +878,7 @@ __global__ void __launch_bounds__(kThreads, 1) window_match_kernel(const __grid_
           const uint32_t r0 = c * q.csteps, steps = min(q.csteps, q.h + 7 - r0);
           const uint32_t a_lo = (ba + s * (L.slot_bytes >> 4)) | (8u << 16);
           if (!MASKED || cc < q.nch) {
-            if (leader) issue_chunk(Chunk{d, a_lo, a_hi, b_lo + r0 * row16, b_hi, row16, q.K, steps, id});
+            if (leader) issue_chunk(Chunk{d, a_lo, a_hi, b_lo + r0 * row16, b_hi, row16, q.K, steps, id, c == 0});
           } else {
             if (!planes_ready) {
               got = mbar_wait(&sh->planes_full, w.ti & 1u, deadline);
@@ -895,16 +890,12 @@ __global__ void __launch_bounds__(kThreads, 1) window_match_kernel(const __grid_
               tc_fence_after();
               planes_ready = true;
               ++ytiles;
-              if (leader) {
-                clear(dy);
-                clear(dy + accw);
-              }
             }
             if (leader)
               for (uint32_t p = 0; p < 2; ++p)
                 issue_chunk(Chunk{dy + p * accw, a_lo, a_hi,
                                   ((pla + p * (L.plane_bytes >> 4)) | (1u << 16)) + r0 * row16, b_hi, row16, q.K, steps,
-                                  id});
+                                  id, c == 0});
           }
           __syncwarp();
           if (leader) {
@@ -1098,13 +1089,12 @@ bool window_plan_for(uint32_t wmax, uint32_t hmax, bool masked, uint32_t nj, uin
   const uint32_t yreg = 16 * nj * kTileW * 4;
   pl.img_off = kFixed + (masked ? std::max(yreg, 2u * pl.plane_bytes) : yreg);
   pl.b_off = pl.img_off + pl.nbuf * pl.plane_bytes;
-  // the template (and mask) as it lies in memory, with slack on both sides
-  // for the blocks' 20-byte reads
-  pl.raw_bytes = (uint32_t)align_up((size_t)wmax * hmax + 96, 128);
+  // the template's (and mask's) rows of K bytes, sixteen zeros ahead
+  pl.raw_bytes = (uint32_t)align_up((size_t)K * hmax + 16, 128);
   const uint32_t raw = pl.raw_bytes * (masked ? 2u : 1u);
   if (pl.b_off + raw >= kSmemMax) return false;
   pl.slot_bytes = (kSmemMax - pl.b_off - raw) / 2 & ~127u;
-  const uint32_t block = 16 * K;
+  const uint32_t block = 16 * K + 32;
   // a template needs no more than a slot of its own size; chunks of fewer than
   // eight steps would build more than they use
   pl.slot_bytes = std::min(pl.slot_bytes, (uint32_t)align_up((size_t)(hmax + 14) * block, 128));
@@ -1118,7 +1108,7 @@ bool window_plan_for(uint32_t wmax, uint32_t hmax, bool masked, uint32_t nj, uin
 // them (its blocks then stay from tile to tile), else one.
 bool window_plan_best(uint32_t wmax, uint32_t hmax, bool masked, uint32_t nj, WindowPlan& pl) {
   if (!masked && window_plan_for(wmax, hmax, masked, nj, 2, pl) &&
-      2 * pl.slot_bytes / (16 * k_of(wmax)) >= hmax + 14)
+      2 * pl.slot_bytes / (16 * k_of(wmax) + 32) >= hmax + 14)
     return true;
   return window_plan_for(wmax, hmax, masked, nj, 1, pl);
 }
@@ -1142,7 +1132,7 @@ WindowProblem window_problem(const MatchArgs& a, const WindowPlan& pl, unsigned 
   // steps 0 .. h + 6 in chunks of csteps, csteps + 7 blocks each: one chunk in
   // a slot, one over both slots (it then stays, but the next template's blocks
   // wait for its last MMA), or as many as it takes
-  const uint32_t block = 16 * q.K, fit = pl.slot_bytes / block, steps = a.h + 7;
+  const uint32_t block = 16 * q.K + 32, fit = pl.slot_bytes / block, steps = a.h + 7;
   q.both = steps + 7 > fit && steps + 7 <= 2 * pl.slot_bytes / block;
   q.nch = q.both ? 1u : (steps + fit - 8) / (fit - 7);
   q.csteps = (steps + q.nch - 1) / q.nch;
