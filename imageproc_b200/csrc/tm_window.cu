@@ -79,6 +79,12 @@ constexpr uint32_t kMmaWarp = kWorkWarps, kLoadWarp = kMmaWarp + 1, kLoadWarps =
 constexpr uint32_t kWarps = kLoadWarp + kLoadWarps, kThreads = kWarps * 32, kLoaders = kLoadWarps * 32;
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kRing = 8;  // tile indices in flight: roles are at most four tiles apart
+// Uses of a block slot that may be complete beyond the one a loader waits for.
+// While a template stays in its slots the MMA warp needs nothing from the
+// loaders but the next tile's image, which they load after they have waited
+// for every use but a slot's last one: at most kMaxSet uses follow.
+constexpr uint32_t kUses = 8;
+static_assert(kUses > kMaxSet + 1, "a slot's uses in flight");
 constexpr uint32_t kHeader = 1024;
 constexpr uint32_t kFixed = kHeader;
 constexpr uint32_t kSmemMax = 227 * 1024;
@@ -114,7 +120,8 @@ __device__ __forceinline__ bool bar_or(uint32_t id, bool fail) {
 
 struct Shared {
   uint64_t img_full[2], img_empty[2];  // image tile slots
-  uint64_t b_full[2], b_empty[2];      // template-block slots
+  uint64_t b_full[2];                  // template-block slots: a chunk is built,
+  uint64_t b_empty[2][kUses];          // ... use n of the slot's blocks is complete (n % kUses)
   uint64_t acc_full[2], acc_empty[2];  // X accumulator buffers
   uint64_t planes_full, yacc_empty;    // masked: the tile's planes of I^2; Y accumulators read
   uint64_t tile_full[kRing];           // tile indices, claimed by the first loader warp
@@ -683,7 +690,7 @@ __global__ void __launch_bounds__(kThreads, 1) window_match_kernel(const __grid_
       mbar_init(&sh->img_full[i], kLoadWarps);
       mbar_init(&sh->img_empty[i], 1 + kWorkWarps);
       mbar_init(&sh->b_full[i], kLoadWarps);
-      mbar_init(&sh->b_empty[i], 1);
+      for (uint32_t u = 0; u < kUses; ++u) mbar_init(&sh->b_empty[i][u], 1);
       mbar_init(&sh->acc_full[i], 1);
       mbar_init(&sh->acc_empty[i], kWorkWarps);
     }
@@ -766,6 +773,9 @@ __global__ void __launch_bounds__(kThreads, 1) window_match_kernel(const __grid_
         __syncwarp();
         if (lane == 0) mbar_arrive(&sh->img_full[slot]);
       };
+      auto wait_use = [&](uint32_t s, uint32_t n) {
+        return mbar_wait_sleep(&sh->b_empty[s][n % kUses], (n / kUses) & 1u, deadline);
+      };
       // a wait that ran out ends the role at the next barrier, in all three
       // warps at once
       bool stop = false;
@@ -791,11 +801,11 @@ __global__ void __launch_bounds__(kThreads, 1) window_match_kernel(const __grid_
         if (resident && m == 0) publish_image();
         for (uint32_t c = 0; c < q.nch * (with_y ? 2u : 1u); ++c) {
           const uint32_t s = q.both ? 0u : (bs.first + c) & 1u;
-          // the slots' last uses first, also where the blocks stay: at most one
-          // use is outstanding, so the barriers' parities say which
+          // the slots' last uses first, also where the blocks stay: every use is
+          // waited for in turn, so the barriers' parities say which
           const bool in0 = !s || q.both, in1 = s || q.both;
-          if (in0 && uses0 && !mbar_wait_sleep(&sh->b_empty[0], (uses0 - 1) & 1u, deadline)) fail = true;
-          if (in1 && uses1 && !mbar_wait_sleep(&sh->b_empty[1], (uses1 - 1) & 1u, deadline)) fail = true;
+          if (in0 && uses0 && !wait_use(0, uses0 - 1)) fail = true;
+          if (in1 && uses1 && !wait_use(1, uses1 - 1)) fail = true;
           uses0 += in0;
           uses1 += in1;
           if (resident) continue;
@@ -830,7 +840,7 @@ __global__ void __launch_bounds__(kThreads, 1) window_match_kernel(const __grid_
   } else if (warp == kMmaWarp) {
     // ---- MMA issue
     BlockState bs;
-    uint32_t builds0 = 0, builds1 = 0, ytiles = 0;
+    uint32_t builds0 = 0, builds1 = 0, uses0 = 0, uses1 = 0, ytiles = 0;
     const bool leader = elect_one();
     const uint32_t imga = smem_u32(img) >> 4, pla = smem_u32(planes) >> 4, ba = smem_u32(bslot) >> 4;
     // test hook: a wait on the drain barrier, which nothing arrives at before the end
@@ -899,9 +909,11 @@ __global__ void __launch_bounds__(kThreads, 1) window_match_kernel(const __grid_
           }
           __syncwarp();
           if (leader) {
-            if (!s || q.both) mma_commit(&sh->b_empty[0]);
-            if (s || q.both) mma_commit(&sh->b_empty[1]);
+            if (!s || q.both) mma_commit(&sh->b_empty[0][uses0 % kUses]);
+            if (s || q.both) mma_commit(&sh->b_empty[1][uses1 % kUses]);
           }
+          uses0 += !s || q.both;
+          uses1 += s || q.both;
           __syncwarp();
         }
         if (fail) break;

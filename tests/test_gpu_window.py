@@ -140,3 +140,36 @@ def test_window_kernel_mixed_group(tune, tmp_path, monkeypatch):
             bad = np.argwhere(bits(out.cpu().numpy()) != bits(want))
             assert bad.size == 0, (sizes[k], bad[:3])
     plan.close()
+
+
+@pytest.mark.parametrize("rows", [16, 32, 64, 128])
+@pytest.mark.parametrize("members", [1, 4])
+def test_window_kernel_short_tiles(rows, members, tmp_path, monkeypatch):
+    # tiles of a few MMAs, many per CTA, of one template that stays in its
+    # slots: the roles run as far ahead of each other as they can
+    import torch
+
+    from imageproc_b200 import _lib, device
+    W, H, w, h = 1920, 1080, 8, 8
+    image, t0, _ = scene(W, H, w, h)
+    pos = (W - w + 1) * (H - h + 1) * members
+    f = tmp_path / "tuning.txt"
+    f.write_text(f"group2 8 0 8 {pos.bit_length() - 1} 10 {100 + members} 0 {rows} {members}\n")
+    monkeypatch.setenv("IPB_TUNING_FILE", str(f))
+    _lib.lib().ipb_batch_tuning_reset()
+    di, dt = torch.from_numpy(image).cuda(), torch.from_numpy(t0).cuda()
+    batch = device.Batch([(di, dt, k) for k in range(members)])
+    plan = device.BatchPlan(batch)
+    assert plan.info()["launches"][0]["tile_rows"] == rows
+    for k in range(20):
+        if k == 19:
+            for o in batch.outs:
+                o.fill_(-1.0)
+        plan.launch()
+    torch.cuda.synchronize()
+    batch.extremes_host()
+    for k, out in enumerate(batch.outs):
+        bad = np.argwhere(bits(out.cpu().numpy()) != bits(O.match_exact(image, t0, k, precision=0)))
+        assert bad.size == 0, (k, bad[:3])
+    plan.close()
+    _lib.lib().ipb_batch_tuning_reset()
