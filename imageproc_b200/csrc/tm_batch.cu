@@ -99,14 +99,13 @@ namespace {
 // Two decisions are tuned and cached per process, and persisted in a text file
 // (IPB_TUNING_FILE, default ~/.cache/imageproc_b200/tuning.txt; an empty
 // IPB_TUNING_FILE keeps them in memory only):
-//  * per batch group (on unless IPB_AUTOTUNE=0): the kernel and its tiles,
-//    timed on the group's own pairs: the Hankel-row kernel's tensor-memory
-//    row width (the group's natural width or twice it), tile height and set
-//    size, or (row width 0) the window kernel's tile rows (plus one: two
-//    image tiles in shared memory) and set size; key = (natural width,
-//    masked, tallest template rounded up to 8, log2 of the group's output
-//    positions, log2 of its largest image side, largest set, plus 100 where
-//    the window kernel was among the candidates).
+//  * per batch group (on unless IPB_AUTOTUNE=0): the launch's tiles, timed on
+//    the group's own pairs: (row width 0) the window kernel's tile rows and
+//    set size where it takes all of the group's pairs, else the Hankel-row
+//    kernel's tensor-memory row width (the group's natural width or twice
+//    it), tile height and set size; key = (natural width, masked, tallest
+//    template rounded up to 8, log2 of the group's output positions, log2 of
+//    its largest image side, largest set, plus 100 for the window kernel).
 //    Line: "group2 ks0 masked h8 wlog mlog set ks nt n".
 //  * per pair shape class (IPB_AUTOTUNE=1): tensor cores or the CUDA-core
 //    kernel, timed on the first pair of each (w, h, masked, normalised).
@@ -271,12 +270,8 @@ ipb_status to_status(cudaError_t e, const char* what) {
     if (e_ != cudaSuccess) return to_status(e_, what); \
   } while (0)
 
-// Times a natural group's launch with each candidate (row width ks0 or
-// 2 ks0, each tile height) on the group's own pairs and returns the fastest.
-// The timing launches write the pairs' outputs and extremes keys; the
-// caller re-arms the keys afterwards.
-// Descriptors of a window-kernel group: rows = tile rows (+ 1 for two image
-// tiles); false when no plan fits.
+// Descriptors of a window-kernel group in tiles of `rows` output rows; false
+// when no plan fits.
 template <class KeysOf>
 bool window_group(const ipb_batch_plan* p, const std::vector<uint32_t>& mem, bool masked, uint32_t rows, uint32_t set,
                   KeysOf keys_of, ipb_batch_plan::Group& g) {
@@ -286,7 +281,8 @@ bool window_group(const ipb_batch_plan* p, const std::vector<uint32_t>& mem, boo
     wmax = std::max(wmax, p->args[i].w);
     hmax = std::max(hmax, p->args[i].h);
   }
-  if (rows < 16 || !window_plan_for(wmax, hmax, masked, rows / 16, 1 + (rows & 1u), g.wplan)) return false;
+  if (rows != 16 && rows != 32 && rows != 64 && rows != 128) return false;
+  if (!window_plan_best(wmax, hmax, masked, rows / 16, g.wplan)) return false;
   g.window = true;
   g.set = set;
   g.wprobs.clear();
@@ -337,9 +333,77 @@ cudaError_t launch_window_group(const ipb_batch_plan* p, const ipb_batch_plan::G
   return launch_window_batch(g.wplan, L, s, t);
 }
 
+// The window kernel's choices for a group: tile rows and set size in order of
+// their estimate, those within 1.25 of the least that have a plan.
+std::vector<GroupChoice> window_choices(const ipb_batch_plan* p, const std::vector<uint32_t>& mem, bool masked,
+                                        uint32_t set) {
+  std::vector<const MatchArgs*> a;
+  uint32_t wmax = 1, hmax = 1;
+  for (uint32_t i : mem) {
+    if (!window_supported(p->args[i])) return {};
+    a.push_back(&p->args[i]);
+    wmax = std::max(wmax, p->args[i].w);
+    hmax = std::max(hmax, p->args[i].h);
+  }
+  std::vector<std::pair<double, GroupChoice>> all;
+  for (uint32_t rows : {128u, 64u, 32u, 16u}) {
+    WindowPlan pl;
+    if (!window_plan_best(wmax, hmax, masked, rows / 16, pl)) continue;
+    all.push_back({window_cost(a.data(), (uint32_t)a.size(), rows / 16, set), GroupChoice{0, rows, set}});
+    if (set > 1) all.push_back({window_cost(a.data(), (uint32_t)a.size(), rows / 16, 1), GroupChoice{0, rows, 1}});
+  }
+  std::stable_sort(all.begin(), all.end(), [](const auto& x, const auto& y) { return x.first < y.first; });
+  std::vector<GroupChoice> c;
+  for (const auto& x : all)
+    if (x.first <= 1.25 * all.front().first) c.push_back(x.second);
+  return c;
+}
+
+// Times the choices on the group's own pairs, in turn, so that a clock that
+// rises meanwhile favours none; one choice needs no timing. The launches write
+// the pairs' outputs and extremes keys; the caller re-arms the keys afterwards.
+template <class KeysOf>
+ipb_status tune_window_group(ipb_batch_plan* p, const std::vector<uint32_t>& mem, bool masked,
+                             const std::vector<GroupChoice>& choices, KeysOf keys_of, GroupChoice& best) {
+  best = choices.front();
+  if (choices.size() == 1) return IPB_OK;
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  IPB_TRY(cudaEventCreate(&e0), "event");
+  if (cudaEventCreate(&e1) != cudaSuccess) {
+    cudaEventDestroy(e0);
+    return to_status(cudaErrorMemoryAllocation, "event");
+  }
+  std::vector<ipb_batch_plan::Group> groups(choices.size());
+  std::vector<float> least(choices.size(), 1e30f);
+  cudaError_t err = cudaSuccess;
+  for (size_t k = 0; k < choices.size() && err == cudaSuccess; ++k) {
+    window_group(p, mem, masked, choices[k].nt, choices[k].set, keys_of, groups[k]);
+    err = upload_window_group(groups[k]);
+  }
+  for (int round = 0; round < 3; ++round)  // the first is a warm-up
+    for (size_t k = 0; k < choices.size() && err == cudaSuccess; ++k) {
+      cudaEventRecord(e0, nullptr);
+      err = launch_window_group(p, groups[k], p->d_sched, false, nullptr, nullptr);
+      cudaEventRecord(e1, nullptr);
+      if (err == cudaSuccess) err = cudaEventSynchronize(e1);
+      float ms = 0;
+      if (err == cudaSuccess && round > 0 && cudaEventElapsedTime(&ms, e0, e1) == cudaSuccess)
+        least[k] = std::min(least[k], ms);
+    }
+  for (auto& g : groups) free_window_group(g);
+  best = choices[std::min_element(least.begin(), least.end()) - least.begin()];
+  cudaEventDestroy(e0);
+  cudaEventDestroy(e1);
+  return to_status(err, "tuning launch");
+}
+
+// Times a natural group's launch with each candidate (row width ks0 or
+// 2 ks0, each tile height) on the group's own pairs and returns the fastest.
+// The timing launches write the pairs' outputs and extremes keys; the
+// caller re-arms the keys afterwards.
 template <class KeysOf>
 ipb_status tune_group(ipb_batch_plan* p, const std::vector<uint32_t>& mem, uint32_t ks0, bool masked, uint32_t hmax,
-                      uint32_t set, bool window, KeysOf keys_of, GroupChoice& best) {
+                      uint32_t set, KeysOf keys_of, GroupChoice& best) {
   best = GroupChoice{ks0, 0, 1};
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   IPB_TRY(cudaEventCreate(&e0), "event");
@@ -396,30 +460,6 @@ ipb_status tune_group(ipb_batch_plan* p, const std::vector<uint32_t>& mem, uint3
       }
     }
    }
-  }
-  if (window) {
-    for (uint32_t sz : sets)
-      for (uint32_t rows : {128u, 129u, 64u, 65u}) {
-        if (masked && (rows & 1u)) continue;  // one image tile only
-        ipb_batch_plan::Group g;
-        if (err != cudaSuccess || !window_group(p, mem, masked, rows, sz, keys_of, g)) continue;
-        err = upload_window_group(g);
-        float ms_best = 1e30f;
-        for (int rep = 0; rep < 3 && err == cudaSuccess; ++rep) {
-          cudaEventRecord(e0, nullptr);
-          err = launch_window_group(p, g, p->d_sched, false, nullptr, nullptr);
-          cudaEventRecord(e1, nullptr);
-          if (err == cudaSuccess) err = cudaEventSynchronize(e1);
-          float ms = 0;
-          if (err == cudaSuccess && rep > 0 && cudaEventElapsedTime(&ms, e0, e1) == cudaSuccess)
-            ms_best = std::min(ms_best, ms);
-        }
-        free_window_group(g);
-        if (err == cudaSuccess && ms_best < best_ms) {
-          best_ms = ms_best;
-          best = GroupChoice{0, rows, sz};
-        }
-      }
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
@@ -691,11 +731,16 @@ ipb_status create(const ipb_pair* pairs, uint32_t n, int precision, bool capture
     const bool masked = p->args[mem.front()].mask != nullptr;
     const uint32_t ks0 = kv.first / 2;  // umma_group_key = row width * 2 + masked
     const uint32_t set = set_of(mem);
-    bool window = kernel_path() == 0;
-    for (uint32_t i : mem) window = window && window_supported(p->args[i]);
+    // the window kernel where it takes every pair: it was the faster one at
+    // every size tried (templates of 8 to 128 pixels a side, images of 512 to
+    // 4096, sets of 1 and 4, masked or not; nearest: 82 against 87 us for one
+    // 32 x 32 template on 4096 x 3000)
+    std::vector<GroupChoice> choices;
+    if (kernel_path() == 0) choices = window_choices(p, mem, masked, set);
+    const bool window = !choices.empty();
     // untuned: sets of up to four unmasked pairs, two binary-mask pairs
     GroupChoice c{ks0, 0, masked ? std::min(set, 2u) : set};
-    if (window) c = GroupChoice{0, 128, set};
+    if (window) c = choices.front();
     if (tune) {
       uint32_t hmax = 0, side = 0;
       double pos = 0;
@@ -718,7 +763,8 @@ ipb_status create(const ipb_pair* pairs, uint32_t n, int precision, bool capture
         }
       }
       if (!have) {
-        ipb_status st = tune_group(p, mem, ks0, masked, hmax, set, window, keys_of, c);
+        ipb_status st = window ? tune_window_group(p, mem, masked, choices, keys_of, c)
+                               : tune_group(p, mem, ks0, masked, hmax, set, keys_of, c);
         if (st != IPB_OK) return fail(st);
         std::lock_guard<std::mutex> lk(g_tune_mu);
         g_group_tune[gk] = c;

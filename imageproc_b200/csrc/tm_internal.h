@@ -333,6 +333,8 @@ struct WindowPlan {
 };
 
 bool window_supported(const MatchArgs& a);
+// Estimated cycles of one launch of n problems; for choosing nj (1, 2, 4, 8) and set.
+double window_cost(const MatchArgs* const* a, uint32_t n, uint32_t nj, uint32_t set);
 // Plan for templates up to wmax x hmax; false when it does not fit.
 bool window_plan_for(uint32_t wmax, uint32_t hmax, bool masked, uint32_t nj, uint32_t nbuf, WindowPlan& pl);
 bool window_plan_best(uint32_t wmax, uint32_t hmax, bool masked, uint32_t nj, WindowPlan& pl);

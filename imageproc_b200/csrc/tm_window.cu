@@ -61,6 +61,7 @@
 // one that runs out records the launch's tag in the error word and the CTA
 // leaves its loops, drains its MMAs and frees its tensor memory.
 #include <algorithm>
+#include <cmath>
 #include <tuple>
 #include <vector>
 
@@ -1248,28 +1249,36 @@ cudaError_t launch_window_batch(const WindowPlan& pl, WindowLaunch& L, cudaStrea
   return cudaGetLastError();
 }
 
-// Tile height of one launch of n problems of one size in sets of up to `set`:
-// the smallest estimate of waves x (the set's MMAs and last epilogue) +
-// set-up, in cycles. An SS MMA of 128 x N x 32 takes max(32 + N/4, N/2); the
-// epilogue about 1000 per 16 output rows.
-uint32_t window_tile_nj(const MatchArgs& a, uint32_t n, uint32_t set) {
-  const uint32_t sms = (uint32_t)device_sm_count(), nsets = (n + set - 1) / set;
-  const uint32_t Wo = a.W - a.w + 1, Ho = a.H - a.h + 1;
-  double best = 0;
-  uint32_t nj_best = 8;
-  for (uint32_t nj : {8u, 4u, 2u, 1u}) {
-    const uint64_t tiles = (uint64_t)((Wo + kTileW - 1) / kTileW) * ((Ho + 16 * nj - 1) / (16 * nj)) * nsets;
-    const double steps = (a.h + 7.0) * std::max(32.0 + 4.0 * nj, 8.0 * nj);
-    const double corr = (double)((n + nsets - 1) / nsets) + (a.mask ? 2.0 : 0.0);
-    const double unit = corr * (k_of(a.w) / 32) * steps + 1000.0 * nj;
-    const double cost = (double)((tiles + sms - 1) / sms) * unit + 6000.0;
-    if (best == 0 || cost < best) {
-      best = cost;
-      nj_best = nj;
-    }
+// Estimated cycles of one launch of n problems in tiles of 16 nj rows and sets
+// of up to `set`: waves of tiles x (a set's MMAs and its epilogues) + set-up.
+// An SS MMA of 128 x N x 32 takes max(32 + N/4, N/2); an epilogue about 1000
+// per 16 output rows. Against 1080p and 512 x 512 maps with templates of 8 to
+// 128 pixels a side the estimate puts the fastest height and set within 1.25
+// of its least (four 64 x 64 templates at 1080p, sets of 4: 128 rows 57 us, 64
+// rows 79; alone: 72 and 85; at 512 x 512, 16 x 16: 27, 20, 17 and 13).
+double window_cost(const MatchArgs* const* a, uint32_t n, uint32_t nj, uint32_t set) {
+  const double sms = (double)device_sm_count(), mma = std::max(32.0 + 4.0 * nj, 8.0 * nj);
+  double tiles = 0, work = 0;
+  for (uint32_t i = 0; i < n; ++i) {
+    const MatchArgs& q = *a[i];
+    const double t = (double)(((q.W - q.w) / kTileW + 1) * (uint64_t)((q.H - q.h) / (16 * nj) + 1));
+    const double corr = 1.0 + (q.mask && q.method != IPB_CROSS_CORRELATION ? 2.0 / set : 0.0);
+    tiles += t / set;
+    work += t * (corr * (k_of(q.w) / 32) * (q.h + 7.0) * mma + 1000.0 * nj);
   }
-  return nj_best;
+  return work / tiles * std::ceil(tiles / sms) + 6000.0;
 }
+
+namespace {
+uint32_t window_tile_nj(const MatchArgs* a, uint32_t n, uint32_t set) {
+  const MatchArgs* p[kInlineProblems];
+  for (uint32_t i = 0; i < n; ++i) p[i] = a + i;
+  uint32_t best = 8;
+  for (uint32_t nj : {4u, 2u, 1u})
+    if (window_cost(p, n, nj, set) < window_cost(p, n, best, set)) best = nj;
+  return best;
+}
+}  // namespace
 
 // One launch of n <= kInlineProblems problems of one image, template size and
 // mask. The image tile is double-buffered when a CTA has several of them and
@@ -1283,7 +1292,7 @@ cudaError_t launch_window_few(const MatchArgs* a, uint32_t n, unsigned long long
   const uint32_t nsets = (n + kMaxSet - 1) / kMaxSet, set = (n + nsets - 1) / nsets;
   WindowPlan pl;
   bool have = false;
-  for (uint32_t nj = window_tile_nj(a[0], n, set); nj >= 1 && !have; nj /= 2)
+  for (uint32_t nj = window_tile_nj(a, n, set); nj >= 1 && !have; nj /= 2)
     have = window_plan_best(a[0].w, a[0].h, a[0].mask != nullptr, nj, pl);
   if (!have) return cudaErrorNotSupported;
   std::vector<WindowProblem> probs(n);
