@@ -46,6 +46,7 @@ using namespace sm100;
 
 constexpr int kM = 128;           // output rows per tile
 constexpr int kXT = 32;           // output columns per tile
+constexpr int kVP = kXT + 1;      // pitch of the row sums: a thread per row, all rows on their own banks
 constexpr int kBuildWarps = 2;
 constexpr int kEpiWarps = 16;  // four per lane quadrant: the epilogue is the longest role
 constexpr int kMmaWarp = kBuildWarps + kEpiWarps;
@@ -89,6 +90,31 @@ __device__ __forceinline__ uint32_t order_key(float f) {
   return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
 }
 
+// n <= 16 bytes at g, zero past them, read as aligned words where those lie
+// inside [p0, end).
+__device__ __forceinline__ uint4 row_chunk(const uint8_t* g, uint32_t n, const uint8_t* p0, const uint8_t* end) {
+  uint32_t v[4] = {0u, 0u, 0u, 0u};
+  const uint32_t off = (uint32_t)(reinterpret_cast<uintptr_t>(g) & 3u);
+  const uint8_t* a = g - off;
+  if (a >= p0 && a + 20 <= end) {
+    const uint32_t* a4 = reinterpret_cast<const uint32_t*>(a);
+    uint32_t w[5];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) w[k] = __ldg(a4 + k);
+    const uint32_t sel = 0x3210u + off * 0x1111u;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      v[k] = __byte_perm(w[k], w[k + 1], sel);
+      if (n < 4u * k + 4u) v[k] = n <= 4u * k ? 0u : v[k] & ((1u << (8 * (n - 4 * k))) - 1u);
+    }
+  } else {
+#pragma unroll
+    for (uint32_t k = 0; k < 16; ++k)
+      if (k < n) v[k >> 2] |= (uint32_t)__ldg(g + k) << (8 * (k & 3));
+  }
+  return make_uint4(v[0], v[1], v[2], v[3]);
+}
+
 // State of an epilogue warp for one tile.
 struct EpiCtx {
   const ManyParams* p;
@@ -98,7 +124,7 @@ struct EpiCtx {
   const uint32_t* s_y;
   const uint32_t* s_tss;
   unsigned long long* s_ext;
-  double* s_ry;  // [kEpiWarps][kPosW] reciprocal roots of the strip's Y (templates as M)
+  double2* s_ry;  // [kEpiWarps][kPosW] {r, -2^52 r}, r the reciprocal root of a position's Y (templates as M)
   uint32_t gx, nx, x0, y0, t0, nt;
   uint32_t e;  // epilogue warp index: lane quadrant (e + kBuildWarps) & 3, share e >> 2
   uint32_t lane;
@@ -124,10 +150,12 @@ __device__ __forceinline__ bool epilogue(EpiCtx& c) {
     // EXACT_FP64 normalisation: 1/sqrt(Y) once per position (shared by the
     // warp's 32 templates) and 1/sqrt(T) once per lane
     constexpr bool kNormW = method_is_norm(kMethod) && kPrec == IPB_PRECISION_EXACT_FP64;
-    double* s_ryw = c.s_ry + c.e * kPosW;
-    const double rT = (kNormW && tss) ? rsqrt_u32(tss) : 0.0;
+    double2* s_ryw = c.s_ry + c.e * kPosW;
+    // lanes past the block's templates write nothing: any factor will do
+    const double rT = !kNormW || !t_ok ? 1.0 : tss ? rsqrt_u32(tss) : 0.0;
     const int mvalid = (int)p.Ho - (int)(c.y0 + mb);  // positions of the share inside the map
-    const size_t rstride = (size_t)p.Wo * p.n;
+    const size_t rstride = (size_t)p.Wo * p.n * 4;  // bytes from row to row
+    const uint32_t lane4 = 4 * c.lane;
     auto score_of = [&](uint32_t v, uint32_t y) -> uint32_t {
       return method_is_sse(kMethod) ? (y + tss - 2u * v) : v;
     };
@@ -137,14 +165,16 @@ __device__ __forceinline__ bool epilogue(EpiCtx& c) {
       tc_fence_after();
       const uint32_t x = c.x0 + xi;
       const uint32_t* ycol = c.s_y + xi * kM + mb;
-      float* ocol = (p.out && t_ok) ? p.out + ((size_t)(c.y0 + mb) * p.Wo + x) * p.n + c.t0 + tl : nullptr;
+      char* ocol = reinterpret_cast<char*>(p.out + ((size_t)(c.y0 + mb) * p.Wo + x) * p.n + c.t0 + q * 32);
+      const bool store = p.out && t_ok;
       // a zero norm anywhere in the share (a window of zeros, or this lane's
       // template all zeros) sends the strip through the general quotient
       bool general = false;
       if constexpr (kNormW) {
         __syncwarp();
         const uint32_t yv = ycol[c.lane];
-        s_ryw[c.lane] = yv ? rsqrt_u32(yv) : 0.0;
+        const double r = yv ? rsqrt_u32(yv) : 0.0;
+        s_ryw[c.lane] = make_double2(r, -4503599627370496.0 * r);
         general = __any_sync(0xffffffffu, yv == 0u) || rT == 0.0;
         __syncwarp();
       }
@@ -153,14 +183,18 @@ __device__ __forceinline__ bool epilogue(EpiCtx& c) {
         if (half >= mvalid) break;  // warp-uniform: past the map's last row
         const int nv = min(16, mvalid - half);
         const uint32_t taddr = tmem_addr(c.tmem, q * 32, d * 128 + mb + half);
-        float* o = ocol ? ocol + (size_t)half * rstride : nullptr;
+        char* o = ocol + (size_t)half * rstride;
         // Fast pass: each value is scored branch-free, stored at once and
         // folded into the half's smallest and largest bits (scores are never
-        // negative, so f32 bits order like the values). FP64 quotients near
-        // an f32 rounding midpoint are flagged.
+        // negative, so f32 bits order like the values). a = RN(s w) is one
+        // fused multiply-add, fma(2^52 + s, w, -2^52 w), with w = ry rT and
+        // -2^52 w = (-2^52 ry) rT, the same rounding at another exponent; it
+        // rounds to f32 by the conversion unit, whose 16 results a cycle leave
+        // the integer unit to the folds. `near` keeps the least distance of
+        // the bits it drops from 256 units below their midpoint: under 512
+        // units some quotient is undecided (norm_bits_fp64_fast's window).
         uint32_t b[16];
-        uint32_t mn = 0xFFFFFFFFu, mx = 0u;
-        bool undecided = false;
+        uint32_t mn = 0xFFFFFFFFu, mx = 0u, near = 0xFFFFFFFFu;
         {
           uint32_t v[16], Y[16];
           tmem_ld16(taddr, v);
@@ -178,9 +212,14 @@ __device__ __forceinline__ bool epilogue(EpiCtx& c) {
 #pragma unroll
             for (int k = 0; k < 16; k += 2) {
               if constexpr (kNormW) {
-                const double2 r2 = *reinterpret_cast<const double2*>(s_ryw + half + k);
-                b[k] = norm_bits_fp64_fast(score_of(v[k], Y[k]), __dmul_rn(r2.x, rT), undecided);
-                b[k + 1] = norm_bits_fp64_fast(score_of(v[k + 1], Y[k + 1]), __dmul_rn(r2.y, rT), undecided);
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                  const double2 r2 = s_ryw[half + k + u];
+                  const double a = __fma_rn(__hiloint2double(0x43300000, (int)score_of(v[k + u], Y[k + u])),
+                                            __dmul_rn(r2.x, rT), __dmul_rn(r2.y, rT));
+                  near = min(near, (uint32_t)__double2loint(a) * 8u + 0x80000800u);
+                  b[k + u] = __float_as_uint(__double2float_rn(a));
+                }
               } else {
                 b[k] = __float_as_uint(finish_score32(kMethod, kPrec, v[k], Y[k], tss));
                 b[k + 1] = __float_as_uint(finish_score32(kMethod, kPrec, v[k + 1], Y[k + 1], tss));
@@ -188,7 +227,8 @@ __device__ __forceinline__ bool epilogue(EpiCtx& c) {
 #pragma unroll
               for (int u = 0; u < 2; ++u)
                 if (kFull || k + u < nv) {
-                  if (o) o[(size_t)(k + u) * rstride] = __uint_as_float(b[k + u]);
+                  if (store)
+                    *reinterpret_cast<float*>(o + (size_t)(k + u) * rstride + lane4) = __uint_as_float(b[k + u]);
                   mn = min(mn, b[k + u]);
                   mx = max(mx, b[k + u]);
                 }
@@ -202,7 +242,7 @@ __device__ __forceinline__ bool epilogue(EpiCtx& c) {
         // Rare and warp-uniform: a half with a flagged or zero-norm quotient
         // reloads its sums, re-scores the flagged values through the general
         // quotient, stores them again and recomputes the half's extremes.
-        if (__any_sync(0xffffffffu, general || undecided)) {
+        if (__any_sync(0xffffffffu, general || near < 0x1000u)) {
           uint32_t v[16];
           tmem_ld16(taddr, v);
           tmem_wait_ld();
@@ -212,12 +252,12 @@ __device__ __forceinline__ bool epilogue(EpiCtx& c) {
               if (k >= nv) break;
               const uint32_t yk = ycol[half + k];
               const uint32_t sk = score_of(v[k], yk);
-              const double w = __dmul_rn(s_ryw[half + k], rT);
+              const double w = __dmul_rn(s_ryw[half + k].x, rT);
               bool u = general;
               if (!general) norm_bits_fp64_fast(sk, w, u);
               if (u) {
                 b[k] = __float_as_uint(norm_quotient_fp64_w(sk, w, yk, tss));
-                if (o) o[(size_t)k * rstride] = __uint_as_float(b[k]);
+                if (store) *reinterpret_cast<float*>(o + (size_t)k * rstride + lane4) = __uint_as_float(b[k]);
               }
             }
           }
@@ -345,7 +385,7 @@ __global__ void __launch_bounds__(kThreads, 1) many_match_kernel(const __grid_co
   uint32_t* s_v = reinterpret_cast<uint32_t*>(smem + p.v_off);   // [rows][kXT]
   unsigned long long* s_ext = reinterpret_cast<unsigned long long*>(smem + p.ext_off);  // [NB][2]
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const uint32_t nch = p.kw / 16;
   const uint32_t strip_bytes = nch * p.rows * 16;
   const uint32_t tb = blockIdx.x % p.nblocks;              // this CTA's template block
@@ -370,31 +410,34 @@ __global__ void __launch_bounds__(kThreads, 1) many_match_kernel(const __grid_co
     tmem_relinquish();
   }
   // template block: chunk (dy, j) holds NB rows of 16 bytes (template t's
-  // bytes [16j, 16j+16) of row dy; zero past w and for absent templates)
-  for (uint32_t idx = threadIdx.x; idx < p.h * nch * p.NB; idx += kThreads) {
-    const uint32_t t = idx % p.NB, c = idx / p.NB;  // c = dy * nch + j
-    const uint32_t dy = c / nch, j = c % nch;
-    uint32_t wd[4] = {0u, 0u, 0u, 0u};
-    if (t < nt) {
-      const uint8_t* row = p.tpl + ((size_t)(t0 + t) * p.h + dy) * p.w;
-#pragma unroll
-      for (int k = 0; k < 16; ++k) {
-        const uint32_t dx = 16 * j + k;
-        if (dx < p.w) wd[k >> 2] |= (uint32_t)__ldg(row + dx) << (8 * (k & 3));
-      }
+  // bytes [16j, 16j+16) of row dy; zero past w and for absent templates).
+  // Eight templates and four chunks per warp: 64 neighbouring bytes of each
+  // are read and 128 of each chunk written. (Byte by byte, a lane per
+  // template, the block of 128 32 x 32 templates took 65 us longer.)
+  {
+    const uint32_t chunks = p.h * nch, c4 = (chunks + 3) / 4, items = c4 * (p.NB / 8);
+    const uint8_t* end = p.tpl + (size_t)p.n * p.w * p.h;
+    for (uint32_t i = warp; i < items; i += kThreads / 32) {
+      const uint32_t c = 4 * (i % c4) + (lane >> 3), t = 8 * (i / c4) + (lane & 7);
+      if (c >= chunks) continue;
+      const uint32_t dy = c / nch, x = 16 * (c % nch);
+      uint4 v = make_uint4(0u, 0u, 0u, 0u);
+      if (t < nt && x < p.w) v = row_chunk(p.tpl + ((size_t)(t0 + t) * p.h + dy) * p.w + x, min(16u, p.w - x), p.tpl, end);
+      *reinterpret_cast<uint4*>(bmat + (size_t)c * p.NB * 16 + t * 16) = v;
     }
-    *reinterpret_cast<uint4*>(bmat + (size_t)c * p.NB * 16 + t * 16) = make_uint4(wd[0], wd[1], wd[2], wd[3]);
   }
+  for (uint32_t t = threadIdx.x; t < p.NB; t += kThreads) s_tss[t] = 0u;
+  __syncthreads();
   // template constants TSS_t = sum T_t^2 (< 2^32 for templates up to 64 x 64)
-  for (uint32_t t = warp; t < p.NB; t += kThreads / 32) {
+  // from the block, its chunks shared out over four threads per template
+  for (uint32_t i = threadIdx.x; i < 4 * p.NB; i += kThreads) {
+    const uint32_t t = i % p.NB;
     uint32_t s = 0;
-    if (t < nt)
-      for (uint32_t k = lane; k < p.w * p.h; k += 32) {
-        const uint32_t v = __ldg(p.tpl + (size_t)(t0 + t) * p.w * p.h + k);
-        s += v * v;
-      }
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if (lane == 0) s_tss[t] = s;
+    for (uint32_t c = i / p.NB; c < p.h * nch; c += 4) {
+      const uint4 v = *reinterpret_cast<const uint4*>(bmat + (size_t)c * p.NB * 16 + t * 16);
+      s = __dp4a(v.x, v.x, __dp4a(v.y, v.y, __dp4a(v.z, v.z, __dp4a(v.w, v.w, s))));
+    }
+    atomicAdd(&s_tss[t], s);
   }
   for (uint32_t i = threadIdx.x; i < 2 * p.NB; i += kThreads) s_ext[i] = (i & 1) ? 0ull : ~0ull;
   fence_proxy_async_smem();
@@ -446,7 +489,7 @@ __global__ void __launch_bounds__(kThreads, 1) many_match_kernel(const __grid_co
       uint32_t s = 0;
       for (uint32_t dx = 0; dx < p.w; ++dx) s += (uint32_t)row[dx] * row[dx];
       for (uint32_t xi = 0; xi < (uint32_t)kXT; ++xi) {
-        s_v[r * kXT + xi] = s;
+        s_v[r * kVP + xi] = s;
         const uint32_t a = row[xi + p.w], b = row[xi];
         s += a * a - b * b;
       }
@@ -455,11 +498,11 @@ __global__ void __launch_bounds__(kThreads, 1) many_match_kernel(const __grid_co
     for (uint32_t idx = threadIdx.x; idx < (uint32_t)kXT * (kM / 32); idx += kThreads) {
       const uint32_t xi = idx % kXT, m0 = (idx / kXT) * 32;
       uint32_t s = 0;
-      for (uint32_t dy = 0; dy < p.h; ++dy) s += (m0 + dy < nrows) ? s_v[(m0 + dy) * kXT + xi] : 0u;
+      for (uint32_t dy = 0; dy < p.h; ++dy) s += (m0 + dy < nrows) ? s_v[(m0 + dy) * kVP + xi] : 0u;
       for (uint32_t m = m0; m < m0 + 32; ++m) {
         s_y[xi * kM + m] = s;
-        const uint32_t a = (m + p.h < nrows) ? s_v[(m + p.h) * kXT + xi] : 0u;
-        const uint32_t b = (m < nrows) ? s_v[m * kXT + xi] : 0u;
+        const uint32_t a = (m + p.h < nrows) ? s_v[(m + p.h) * kVP + xi] : 0u;
+        const uint32_t b = (m < nrows) ? s_v[m * kVP + xi] : 0u;
         s += a - b;
       }
     }
@@ -541,7 +584,7 @@ __global__ void __launch_bounds__(kThreads, 1) many_match_kernel(const __grid_co
         atomicMax(p.err, p.tag);
       }
     } else {
-      EpiCtx c{&p, tmem, dfull, dempty, s_y, s_tss, s_ext, reinterpret_cast<double*>(smem + p.ry_off),
+      EpiCtx c{&p, tmem, dfull, dempty, s_y, s_tss, s_ext, reinterpret_cast<double2*>(smem + p.ry_off),
                gx, nx, x0, y0, t0, nt,
                (uint32_t)(warp - kBuildWarps), (uint32_t)lane, deadline, kmin, kmax};
       ok = epilogue<kTplM, kMethod, kPrec, kExt>(c);
@@ -620,9 +663,9 @@ uint32_t many_carve(ManyParams& p, uint32_t nb) {
   p.y_off = off;
   off += kXT * kM * 4;
   p.v_off = off;
-  off += (uint32_t)align_up((size_t)p.rows * kXT * 4, 128);
+  off += (uint32_t)align_up((size_t)p.rows * kVP * 4, 128);
   p.ry_off = off;
-  off += kEpiWarps * kPosW * 8;
+  off += kEpiWarps * kPosW * 16;
   return off;
 }
 

@@ -239,7 +239,7 @@ def match_templates_device(image: torch.Tensor, templates: torch.Tensor, method,
     ex = None
     if extremes:
         import numpy as np
+        # the records as tuples at once: field by field they cost 3 us each
         raw = ext.cpu().numpy().view(np.dtype(EXTREMES_DTYPE)).reshape(-1)
-        ex = [Extremes(float(r["max_value"]), float(r["min_value"]), (int(r["max_x"]), int(r["max_y"])),
-                       (int(r["min_x"]), int(r["min_y"]))) for r in raw]
+        ex = [Extremes(mx, mn, (xx, xy), (nx, ny)) for mx, mn, xx, xy, nx, ny in raw.tolist()]
     return (out if scores else None), ex
