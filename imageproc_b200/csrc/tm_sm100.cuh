@@ -70,6 +70,23 @@ __device__ __forceinline__ bool mbar_wait_sleep(uint64_t* bar, uint32_t parity, 
   return true;
 }
 
+// Barrier of kCount threads that also tells every one of them whether any
+// passed `fail` (so a wait that ran out in one warp ends the role in all).
+template <int kCount>
+__device__ __forceinline__ bool bar_or(uint32_t id, bool fail) {
+  uint32_t r;
+  __syncwarp();
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "bar.red.or.pred q, %2, %3, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(r)
+      : "r"((uint32_t)fail), "r"(id), "n"(kCount)
+      : "memory");
+  return r != 0;
+}
+
 // ---- proxy / tcgen05 ordering ------------------------------------------------
 // Generic-proxy writes to shared memory made visible to the async proxy (the
 // tensor core reads its B operand through it).

@@ -102,23 +102,6 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
                : "memory");
 }
 
-// Barrier of kCount threads that also tells every one of them whether any
-// passed `fail` (so a wait that ran out in one warp ends the role in all).
-template <int kCount>
-__device__ __forceinline__ bool bar_or(uint32_t id, bool fail) {
-  uint32_t r;
-  __syncwarp();
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.u32 p, %1, 0;\n\t"
-      "bar.red.or.pred q, %2, %3, p;\n\t"
-      "selp.u32 %0, 1, 0, q;\n\t}"
-      : "=r"(r)
-      : "r"((uint32_t)fail), "r"(id), "n"(kCount)
-      : "memory");
-  return r != 0;
-}
-
 struct Shared {
   uint64_t img_full[2], img_empty[2];  // image tile slots
   uint64_t b_full[2];                  // template-block slots: a chunk is built,

@@ -67,6 +67,38 @@ def test_many_templates_bit_exact(case):
                 (float(mx), float(mn), mxl, mnl), (t, method)
 
 
+# (H, W), (n, h, w): the bank in tensor memory at the edges of its units: one,
+# three and an even number of 16-byte chunks per row with rows that have and
+# have no partner, 1, 32 and 33 units, banks that fill and overflow a block,
+# maps of one row, one column, one position, a tile of 128 rows and one more
+BANK_CASES = [
+    ((128, 160), (65, 1, 16)), ((131, 90), (128, 4, 16)), ((200, 101), (70, 37, 16)), ((160, 47), (66, 33, 17)),
+    ((300, 130), (129, 32, 32)), ((290, 64), (100, 33, 32)), ((90, 256), (80, 21, 33)), ((150, 120), (68, 22, 48)),
+    ((64, 300), (90, 23, 47)), ((17, 64), (128, 17, 64)), ((140, 49), (72, 13, 49)), ((40, 36), (65, 40, 36)),
+]
+
+
+@pytest.mark.parametrize("case", BANK_CASES, ids=lambda c: f"{c[0][0]}x{c[0][1]}_n{c[1][0]}_{c[1][1]}x{c[1][2]}")
+def test_bank_in_tensor_memory(case):
+    (H, W), (n, h, w) = case
+    g = np.random.default_rng(H + 7 * n)
+    image = g.integers(0, 256, (H, W), dtype=np.uint8)
+    image[: H // 2, : W // 3] = 0  # zero norms
+    templates = g.integers(0, 256, (n, h, w), dtype=np.uint8)
+    templates[n // 2] = 0
+    for method, prec in ((M.CrossCorrelationNormalized, 0), (M.SumOfSquaredErrorsNormalized, 0),
+                         (M.CrossCorrelation, 0), (M.SumOfSquaredErrorsNormalized, 1)):
+        out, ex = _run(image, templates, method, tm.Precision(prec))
+        for t in sorted({0, 1, 31, 32, n // 2, n - 1}):
+            exp = O.match_exact(image, templates[t], method, None, precision=prec)
+            bad = np.argwhere(bits(out[:, :, t]) != bits(exp))
+            assert bad.size == 0, (t, method, bad[:3])
+            mx, mn, mxl, mnl = O.find_extremes(exp)
+            e = ex[t]
+            assert (e.max_value, e.min_value, e.max_value_location, e.min_value_location) == \
+                (float(mx), float(mn), mxl, mnl), (t, method)
+
+
 @pytest.mark.parametrize("n", [20, 100])  # positions as M, templates as M
 def test_many_templates_extremes_ties_first_occurrence(n):
     # a periodic scene: every template's best (and worst) score repeats every
