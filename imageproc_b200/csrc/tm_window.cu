@@ -52,9 +52,10 @@
 // sums.
 //
 // Roles (20 warps): sixteen workers, one MMA warp, three loader warps (image
-// tile by one tensor copy; template blocks, built in chunks of template
-// rows into two slots, so a template of any height streams through; a
-// template that fits the slots stays for the following tiles of its problem).
+// tile by one tensor copy where its rows allow one, else the workers load it;
+// template blocks, built in chunks of template rows into two slots, so a
+// template of any height streams through; a template that fits the slots stays
+// for the following tiles of its problem).
 // Before the roles part, all warps load the CTA's first tile and build its
 // first blocks. The X accumulators are double-buffered, the image tile where
 // shared memory allows. Every wait is bounded;
@@ -235,7 +236,7 @@ __device__ __forceinline__ void load_tensor(const CUtensorMap* map, bool global,
                                             uint32_t bytes, uint64_t* bar) {
   if (global) asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(map) : "memory");
   mbar_arrive_expect_tx(bar, bytes);
-  for (uint32_t i = 1; i < kLoadWarps; ++i) mbar_arrive(bar);
+  for (uint32_t i = 1; i < kWorkWarps; ++i) mbar_arrive(bar);
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::
           "r"(smem_u32(dst)),
@@ -671,7 +672,7 @@ __global__ void __launch_bounds__(kThreads, 1) window_match_kernel(const __grid_
   set_tile(w, L, P, blockIdx.x);
   if (tid == kLoadWarp * 32) {
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&sh->img_full[i], kLoadWarps);
+      mbar_init(&sh->img_full[i], kWorkWarps);
       mbar_init(&sh->img_empty[i], 1 + kWorkWarps);
       mbar_init(&sh->b_full[i], kLoadWarps);
       for (uint32_t u = 0; u < kUses; ++u) mbar_init(&sh->b_empty[i][u], 1);
@@ -734,28 +735,22 @@ __global__ void __launch_bounds__(kThreads, 1) window_match_kernel(const __grid_
       const uint32_t slot = L.nbuf == 2 ? (w.ti & 1u) : 0u;
       uint8_t* dst = img + slot * L.plane_bytes;
       const bool by_tensor = P[w.pi].load_mode == 2, need_y = P[w.pi].need_y;
+      // one tensor copy, where the rows allow it; the workers load other
+      // images. The slot's last tile is waited for either way: every phase in
+      // turn, so that the parity says which.
       auto load = [&]() {
         const uint32_t use = w.ti / L.nbuf;  // earlier tiles in this slot
-        if (by_tensor && lw) return;  // the first loader warp's
+        if (lw) return;
         bool got = true;
         if (use) got = mbar_wait_sleep(&sh->img_empty[slot], (use - 1) & 1u, deadline);
         if (!__all_sync(0xffffffffu, got)) {
           fail = true;
-        } else if (by_tensor) {
-          if (lane == 0) load_tensor(maps + w.pi, !inl, w, dst, P[w.pi].tile_bytes, &sh->img_full[slot]);
-          __syncwarp();
-          (slot ? last1 : last0) = (int)use;
-        } else {
-          load_image(P[w.pi], w, dst, lt, kLoaders);
-          (slot ? last1 : last0) = -1;
+          return;
         }
-      };
-      auto publish_image = [&]() {
-        if (by_tensor) return;
-        cp_async_wait_all();
-        fence_proxy_async_smem();
+        (slot ? last1 : last0) = by_tensor ? (int)use : -1;
+        if (by_tensor && lane == 0)
+          load_tensor(maps + w.pi, !inl, w, dst, P[w.pi].tile_bytes, &sh->img_full[slot]);
         __syncwarp();
-        if (lane == 0) mbar_arrive(&sh->img_full[slot]);
       };
       auto wait_use = [&](uint32_t s, uint32_t n) {
         return mbar_wait_sleep(&sh->b_empty[s][n % kUses], (n / kUses) & 1u, deadline);
@@ -782,7 +777,6 @@ __global__ void __launch_bounds__(kThreads, 1) window_match_kernel(const __grid_
           }
           add_tss(raw, q.h * (q.K / 4), tss, lt, kLoaders);
         }
-        if (resident && m == 0) publish_image();
         for (uint32_t c = 0; c < q.nch * (with_y ? 2u : 1u); ++c) {
           const uint32_t s = q.both ? 0u : (bs.first + c) & 1u;
           // the slots' last uses first, also where the blocks stay: every use is
@@ -803,10 +797,7 @@ __global__ void __launch_bounds__(kThreads, 1) window_match_kernel(const __grid_
             __syncwarp();
           }
           if (lane == 0) mbar_arrive(&sh->b_full[s]);
-          if (c == 0 && m == 0) {
-            if (!first && L.nbuf == 1) load();
-            publish_image();
-          }
+          if (c == 0 && m == 0 && !first && L.nbuf == 1) load();
         }
       }
       if (stop) {
@@ -815,7 +806,6 @@ __global__ void __launch_bounds__(kThreads, 1) window_match_kernel(const __grid_
       }
     }
     // no copy is in flight when the CTA leaves
-    cp_async_wait_all();
     if (lw == 0) {
       const unsigned long long deadline = global_ns() + kDefaultWaitNs;
       if (last0 >= 0) mbar_wait_sleep(&sh->img_full[0], last0 & 1, deadline);
@@ -931,6 +921,7 @@ __global__ void __launch_bounds__(kThreads, 1) window_match_kernel(const __grid_
     const uint32_t quad = warp & 3, sub = warp >> 2;
     const uint32_t g0 = sub * 2 * nj / 4, g1 = (sub + 1) * 2 * nj / 4;
     const bool together = MASKED || nj == 1;
+    if (P[w.pi].load_mode != 2 && lane == 0) mbar_arrive(&sh->img_full[0]);  // the first tile, loaded by all
     uint32_t tss = 0, tss_of = 0xFFFFFFFFu;  // sum (T m)^2 and the problem it is of
     for (;; ++w.ti) {
       const unsigned long long deadline = global_ns() + L.wait_ns;
@@ -974,15 +965,43 @@ __global__ void __launch_bounds__(kThreads, 1) window_match_kernel(const __grid_
         break;
       }
       if (!more) break;
+      // The next tile's image, where no tensor copy takes it: by all workers
+      // (three loader warps took 2.5 us longer per tile, on which the MMAs
+      // waited: 60 uneven maps, 57 of them with rows on odd addresses, 1365
+      // us), once the slot is free: with one slot when the last member's MMAs
+      // are done, before its epilogue, which then runs beside the next MMAs.
+      auto load_next = [&]() {
+        Walk nx = w;
+        ++nx.ti;
+        const bool have = next_tile<false>(nx, L, P, sh, deadline);
+        if (!__all_sync(0xffffffffu, nx.ok)) fail = true;
+        if (fail || !have || P[nx.pi].load_mode == 2) return;
+        const uint32_t ns = L.nbuf == 2 ? (nx.ti & 1u) : 0u, use = nx.ti / L.nbuf;
+        bool free = true;
+        if (use) free = mbar_wait_sleep(&sh->img_empty[ns], (use - 1) & 1u, deadline);
+        if (!__all_sync(0xffffffffu, free)) {
+          fail = true;
+          return;
+        }
+        load_image(P[nx.pi], nx, img + ns * L.plane_bytes, tid, kWorkWarps * 32);
+        cp_async_wait_all();
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sh->img_full[ns]);
+      };
       for (uint32_t m = 0; m < w.nset && !fail; ++m, ++w.it) {
         const WindowProblem& q = P[w.pi + m];
         const uint32_t buf = w.it & 1u;
+        // not before the last member: the loaders claim the next tile when
+        // they have built the last one's blocks
+        if (L.nbuf == 2 && m + 1 == w.nset) load_next();
         const bool got = mbar_wait_sleep(&sh->acc_full[buf], (w.it >> 1) & 1u, deadline);
-        if (!__all_sync(0xffffffffu, got)) {
+        if (!__all_sync(0xffffffffu, got && !fail)) {
           fail = true;
           break;
         }
         tc_fence_after();
+        if (L.nbuf == 1 && m + 1 == w.nset) load_next();
         // a template that follows itself may have stayed in its slots; its sum
         // is then not handed over again
         if (tss_of == 0xFFFFFFFFu || P[tss_of].tpl != q.tpl || P[tss_of].mask != q.mask || P[tss_of].w != q.w ||
