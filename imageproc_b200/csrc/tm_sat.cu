@@ -152,15 +152,37 @@ __global__ void __launch_bounds__(32 * kSegs) sat_cols_kernel(uint32_t cols, uin
 
 constexpr uint32_t kStripRows = 16, kTileCols = 1024, kTileThreads = 256;
 
-// The four pixels of a thread, zero past the image: one word where rows are
-// word-aligned.
-__device__ __forceinline__ uint32_t four_pixels(const uint8_t* __restrict__ row, uint32_t x, uint32_t W, bool aligned) {
-  if (aligned && x + 4 <= W) return __ldg(reinterpret_cast<const uint32_t*>(row + x));
-  uint32_t v = 0;
+// A thread's four pixels at x of each of a strip's first n rows, zero past the
+// image: one word per row where rows are word-aligned, else the two aligned
+// words around them, without a branch between the rows' loads (with one, or
+// byte by byte, the rows' latencies added up and odd widths were slower than
+// by a pass per row and one per column); by bytes in the strips at the image's
+// ends, where the words would leave it.
+__device__ __forceinline__ void strip_pixels(const uint8_t* __restrict__ img, uint32_t W, uint32_t H, uint32_t y0,
+                                             uint32_t n, uint32_t x, bool aligned, uint32_t (&v)[kStripRows]) {
+  const uint8_t* p = img + (size_t)y0 * W + min(x, W - 1);
+  const uint32_t in = x < W ? min(4u, W - x) : 0u, mask = in < 4 ? (1u << (8 * in)) - 1u : 0xFFFFFFFFu;
+  if (aligned) {
 #pragma unroll
-  for (uint32_t k = 0; k < 4; ++k)
-    if (x + k < W) v |= (uint32_t)__ldg(row + x + k) << (8 * k);
-  return v;
+    for (uint32_t r = 0; r < kStripRows; ++r)
+      v[r] = r < n && in ? __ldg(reinterpret_cast<const uint32_t*>(p + (size_t)r * W)) : 0u;
+  } else if (y0 && y0 + kStripRows < H) {
+#pragma unroll
+    for (uint32_t r = 0; r < kStripRows; ++r) {
+      const uint8_t* g = p + (size_t)r * W;
+      const uint32_t off = (uint32_t)(reinterpret_cast<uintptr_t>(g) & 3u);
+      const uint32_t* w = reinterpret_cast<const uint32_t*>(g - off);
+      v[r] = __byte_perm(__ldg(w), __ldg(w + 1), 0x3210u + off * 0x1111u) & mask;
+    }
+  } else {
+#pragma unroll
+    for (uint32_t r = 0; r < kStripRows; ++r) {
+      v[r] = 0;
+#pragma unroll
+      for (uint32_t k = 0; k < 4; ++k)
+        if (r < n && k < in) v[r] |= (uint32_t)__ldg(p + (size_t)r * W + k) << (8 * k);
+    }
+  }
 }
 template <bool kSquare>
 __device__ __forceinline__ uint32_t term(uint32_t v, int k) {
@@ -185,9 +207,7 @@ __global__ void __launch_bounds__(kTileThreads) sat_strip_sums_kernel(const uint
     for (uint32_t tile = 0; tile < W; tile += kTileCols) {
       const uint32_t x = tile + 4 * threadIdx.x;
       uint32_t v[kStripRows], c[4] = {0u, 0u, 0u, 0u};
-#pragma unroll
-      for (uint32_t r = 0; r < kStripRows; ++r)
-        v[r] = r < rows && x < W ? four_pixels(img + (size_t)(y0 + r) * W, x, W, aligned) : 0u;
+      strip_pixels(img, W, H, y0, rows, x, aligned, v);
 #pragma unroll
       for (uint32_t r = 0; r < kStripRows; ++r) {
         uint32_t t;
@@ -290,9 +310,7 @@ __global__ void __launch_bounds__(kTileThreads) sat_tiles_kernel(const uint8_t* 
   const uint32_t form = rows == kStripRows ? kStripRows - 1 : rows;  // the whole strip's last row is final
   const uint32_t x = tile + 4 * threadIdx.x;
   uint32_t v[kStripRows];
-#pragma unroll
-  for (uint32_t r = 0; r < kStripRows; ++r)
-    v[r] = r < form && x < W ? four_pixels(img + (size_t)(y0 + r) * W, x, W, aligned) : 0u;
+  strip_pixels(img, W, H, y0, form, x, aligned, v);
   // the row above the strip, in the columns this thread stores
   T base[4];
 #pragma unroll
@@ -396,8 +414,18 @@ cudaError_t launch_sat_typed(const uint8_t* img, uint32_t W, uint32_t H, T* sat,
   if (e != cudaSuccess || H == 0) return e;
   if (W == 0) return cudaMemsetAsync(sat, 0, sizeof(T) * (size_t)cols * (H + 1), s);
   if constexpr (C == 1) {
-    // tiles are counted in 31 bits
-    if ((uint64_t)((H + kStripRows - 1) / kStripRows) * ((W + kTileCols - 1) / kTileCols) < 0x7FFFFFFFull)
+    // One block per strip sums it tile after tile, so with few strips the SMs
+    // stand idle and the row pass, a block per row, is the faster one; rows
+    // that are not word-aligned cost the strips two words per four pixels,
+    // twice. u64 squares, row and column pass against this: 512 x 2048 16.8
+    // and 21.2 us, 900 x 2048 24.8 and 21.1, 1024 x 4096 29.5 and 30.3, 1500
+    // x 4096 42.5 and 34, 4096 x 4096 117 and 60; 1500 x 2047 29.6 and 32.6,
+    // 2111 x 4095 50.7 and 50.3, 3333 x 4095 86 and 80. Tiles are counted in
+    // 31 bits.
+    const uint32_t strips = H / kStripRows, tiles_x = (W + kTileCols - 1) / kTileCols;
+    const bool words = W % 4 == 0 && (reinterpret_cast<uintptr_t>(img) & 3u) == 0;
+    if (strips >= (words ? 72 + 4 * tiles_x : 100 + 25 * tiles_x) &&
+        (uint64_t)(strips + 1) * tiles_x < 0x7FFFFFFFull)
       return launch_sat_one_channel<T, kSquare>(img, W, H, sat, s);
   }
   sat_rows_kernel<T, kSquare, C><<<H < 65535u ? H : 65535u, kRowThreads, 0, s>>>(img, W, H, sat);

@@ -52,6 +52,15 @@ def test_integral_tiles(W, H, dtype):
         assert np.array_equal(got, exp.astype(dtype))
 
 
+@pytest.mark.parametrize("dtype", [np.uint32, np.uint64])
+@pytest.mark.parametrize("W,H", [(4, 1215), (4, 1216), (1024, 1231), (1028, 1283), (2052, 1361), (1, 2000), (3, 2017),
+                                 (1023, 2015), (1025, 2401), (2049, 2800)])
+def test_integral_strips(W, H, dtype):
+    # tall enough for the strips: rows on and off word boundaries, whole and
+    # partial last strips, columns at a tile's edges
+    test_integral_tiles(W, H, dtype)
+
+
 def test_integral_unaligned_device_buffers_and_capture():
     # rows off word boundaries, a poisoned table, and the call inside a graph
     import torch
