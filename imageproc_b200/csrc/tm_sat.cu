@@ -21,7 +21,7 @@
 // one exchange between warps per row, staged in 32 bits so that warps store
 // contiguous runs). Nothing but the table holds intermediates. The bound is
 // the table's one write: 4096 x 4096 squared u64, 23 us for image and table
-// at the copy rate; two passes over the table 117 us, this 65 us.
+// at the copy rate; two passes over the table 117 us, this 60 us.
 //
 // Three and four channels: two passes over the table: a row scan (one block
 // per row, tiles of 1024 pixels scanned block-wide and stored through shared

@@ -968,7 +968,7 @@ __global__ void __launch_bounds__(kThreads, 1) window_match_kernel(const __grid_
       // The next tile's image, where no tensor copy takes it: by all workers
       // (three loader warps took 2.5 us longer per tile, on which the MMAs
       // waited: 60 uneven maps, 57 of them with rows on odd addresses, 1365
-      // us), once the slot is free: with one slot when the last member's MMAs
+      // us, so 1000), once the slot is free: with one slot when the last member's MMAs
       // are done, before its epilogue, which then runs beside the next MMAs.
       auto load_next = [&]() {
         Walk nx = w;
