@@ -653,7 +653,10 @@ __global__ void __launch_bounds__(256) certify_l2_kernel(const uint8_t* __restri
 // Level 3: the 16 micro blocks (4 x 4 positions) inside each list2 entry. A
 // micro block that is neither excluded nor inside a verified window is
 // appended to the template's extra list (counter n_extra[t]); a count above
-// kMaxExtra means the template falls back.
+// kMaxExtra means the template falls back. The counter is a result: every
+// block is counted, also past the cap, whatever the order in which the
+// launch's blocks run (a template whose level-2 list overflowed keeps the
+// kMaxExtra + 1 recorded there).
 __global__ void __launch_bounds__(256) certify_l3_kernel(const uint8_t* __restrict__ tpl,
                                                          const TopK* __restrict__ tk, float min_margin,
                                                          const unsigned long long* __restrict__ best,
@@ -671,8 +674,8 @@ __global__ void __launch_bounds__(256) certify_l3_kernel(const uint8_t* __restri
   if (threadIdx.x < nw) s_win[threadIdx.x] = wins[(size_t)t * max_rects + threadIdx.x];
   CertCtx cc;
   cert_setup(cc, s_st, tpl + (size_t)t * kTpl * kTpl, tk[t], min_margin, best[t]);  // syncs s_win too
-  if (cc.skip || n_extra[t] > (uint32_t)kMaxExtra) return;
-  const uint32_t work = min(n2[t], kMaxLevel2) * 16u;
+  if (cc.skip || n2[t] > kMaxLevel2) return;
+  const uint32_t work = n2[t] * 16u;
   for (uint32_t e = blockIdx.y * blockDim.x + threadIdx.x; e < work; e += gridDim.y * blockDim.x) {
     const uint32_t p2 = list2[(size_t)t * kMaxLevel2 + (e >> 4)], k1 = e & 15u;
     const uint32_t px = p2 % Pmx + (k1 & 3), py = p2 / Pmx + (k1 >> 2);

@@ -430,7 +430,8 @@ typedef struct ipb_proposal_result {
     uint32_t path;      /* 0: proposals, verified and certified; 1: fallback (low margin);
                            2: fallback (not certified) */
     uint32_t uncertified; /* blocks of 4 x 4 positions the certificate could not exclude
-                             outside the proposed windows (verified exactly when at most 16384) */
+                             outside the proposed windows (verified exactly when at most 16384);
+                             16385 where more than 65536 of its blocks of 16 x 16 positions stayed */
 } ipb_proposal_result;
 
 /* Answers n_templates SumOfSquaredErrors queries of 48 x 48 templates

@@ -165,6 +165,29 @@ def test_ablation_network_and_pyramid_proposals():
     assert all(a.path in (0, 2) for a in net0 + pyr)  # no margin gate on these
 
 
+def test_uncertified_counts_above_the_verified_limit():
+    # a flat scene and flat templates: every bound equals the score, so no block
+    # outside the window is excluded and the count is known: all blocks of 4 x 4
+    # positions but the window's. 64 templates are more thread blocks than run
+    # at once, and each must count all of its own. 1024 x 1024 is over the 16384
+    # blocks that are verified, 4160 x 4160 over the 65536 blocks of 16 x 16 of a
+    # template's list.
+    import torch
+    for side, origin, fixed in ((1024, 400 * 977 + 400, None), (4160, 0, 16385)):
+        image = torch.full((side, side), 90, dtype=torch.uint8, device="cuda")
+        templates = torch.arange(64, dtype=torch.uint8, device="cuda").view(64, 1, 1).expand(64, 48, 48).contiguous()
+        origins = torch.full((64, 1), origin, dtype=torch.int32, device="cuda")
+        blocks = ((side - 47 + 3) // 4) ** 2
+        assert fixed is None or ((side - 47 + 15) // 16) ** 2 > 65536
+        expected = blocks - 8 * 8 if fixed is None else fixed  # the 32 x 32 window at (384, 384)
+        for _ in range(3):
+            answers = learned.match_proposals(image, templates, origins)
+            assert [a.uncertified for a in answers] == [expected] * 64
+            assert [a.path for a in answers] == [2] * 64
+            assert [a.location for a in answers] == [(0, 0)] * 64
+            assert [a.value for a in answers] == [float(2304 * (90 - k) ** 2) for k in range(64)]
+
+
 def test_rejects_unsupported_queries():
     import torch
     net = learned.ProposalNet(seed=1)
