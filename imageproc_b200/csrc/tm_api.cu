@@ -193,7 +193,7 @@ struct DevBuf {
 struct Context {
   int device = -1;
   cudaStream_t stream = nullptr;
-  cudaEvent_t last = nullptr;  // last use of any scratch buffer below
+  cudaEvent_t last = nullptr;  // last launch, and last use of any scratch buffer below
   DevBuf scratch, ext_scratch, img, tpl, mask, out;
   void* pinned = nullptr;  // small pinned host block: reduction results, error words
   DevBuf errw;                     // tensor-core error word (largest failing launch tag)
@@ -335,6 +335,13 @@ ipb_status finish_sync(Context* c, cudaStream_t s, bool err_copied = false) {
   return IPB_OK;
 }
 
+bool is_capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
+  (void)cudaGetLastError();  // the null stream beside a capture: the calls below report it
+  return false;
+}
+
 // Enqueue one matching problem on a.stream.
 ipb_status run_match(Context* c, const MatchArgs& a) {
   const size_t out_bytes = (size_t)(a.W - a.w + 1) * (a.H - a.h + 1) * sizeof(float);
@@ -360,8 +367,12 @@ ipb_status run_match(Context* c, const MatchArgs& a) {
     const size_t need = ref ? reference_scratch_bytes(a) : exact_cc_scratch_bytes(a);
     if ((st = ensure(c, c->scratch, need))) return st;
   }
-  // a window launch uses no scratch, only the error word (set by atomics)
-  if (!window) IPB_CUDA(cudaStreamWaitEvent(a.stream, c->last, 0), "cudaStreamWaitEvent");
+  // Every launch follows the context's last one and is its last one then, so
+  // that a synchronising call on any stream waits for all of them before it
+  // reads the error word. A window launch uses no scratch and may be recorded
+  // into a graph; it runs with the graph and takes no part in that order.
+  const bool recorded = window && is_capturing(a.stream);
+  if (!recorded) IPB_CUDA(cudaStreamWaitEvent(a.stream, c->last, 0), "cudaStreamWaitEvent");
   MatchArgs la = a;
   la.timer = acquire_timer();
   cudaError_t e;
@@ -383,7 +394,7 @@ ipb_status run_match(Context* c, const MatchArgs& a) {
                (double)a.W * a.H + tp * (a.mask ? 2.0 : 1.0) + 4.0 * Wo * Ho);
   }
   if (e != cudaSuccess) return cuda_fail(e, "template-matching launch");
-  if (!window) IPB_CUDA(cudaEventRecord(c->last, a.stream), "cudaEventRecord");
+  if (!recorded) IPB_CUDA(cudaEventRecord(c->last, a.stream), "cudaEventRecord");
   return IPB_OK;
 }
 

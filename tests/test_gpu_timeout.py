@@ -89,3 +89,59 @@ def test_many_templates_wait_runs_out_then_context_recovers(tiny_budget):
     k = 77
     exp = O.match_exact(image, templates[k], 3, None, precision=0)
     assert np.array_equal(bits(out[:, :, k].cpu().numpy()), bits(exp))
+
+
+@pytest.mark.parametrize("sync", ["extremes", "host_match"])
+def test_timeout_on_another_stream_is_reported(tiny_budget, sync):
+    # the failing launch is behind enough work on its stream that a call which
+    # did not wait for it would read the error word first
+    import torch
+
+    from imageproc_b200 import device
+    L = tiny_budget
+    image, template, _, _ = synthetic.blob_scene(W=700, H=400, tw=64, th=48, seed=78)
+    di, dt = torch.from_numpy(image).cuda(), torch.from_numpy(template).cuda()
+    scores, out = torch.rand((64, 64), device="cuda"), torch.empty((400 - 47, 700 - 63), device="cuda")
+    tm.set_precision(tm.Precision.ExactFp64)
+    tm.set_path(tm.Path.Auto)
+    busy = torch.empty(1 << 28, dtype=torch.uint8, device="cuda")
+
+    def wait_on_other_stream():
+        if sync == "extremes":
+            device.find_extremes_device(scores, stream=other)
+        else:
+            tm.match_template(image, template, 0)
+
+    stream, other = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    wait_on_other_stream()  # buffers grown: nothing below waits for the device
+    with torch.cuda.stream(stream):
+        for _ in range(100):
+            busy.zero_()
+        _stall(L, True)
+        device.match_template_device(di, dt, 0, out=out)
+        _stall(L, False)
+    with pytest.raises(_lib.DeviceError, match=r"status 9\].*timed out"):
+        wait_on_other_stream()
+    torch.cuda.synchronize()
+    wait_on_other_stream()  # reported once
+
+
+def test_match_recorded_into_a_graph():
+    import torch
+
+    from imageproc_b200 import device
+    image, template, _, _ = synthetic.blob_scene(W=700, H=400, tw=64, th=48, seed=79)
+    di, dt = torch.from_numpy(image).cuda(), torch.from_numpy(template).cuda()
+    out = torch.empty((400 - 47, 700 - 63), device="cuda")
+    tm.set_precision(tm.Precision.ExactFp64)
+    tm.set_path(tm.Path.Auto)
+    device.match_template_device(di, dt, 3, out=out)  # buffers grown, a launch on the context's record
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        device.match_template_device(di, dt, 3, out=out)
+    out.zero_()
+    graph.replay()
+    tm.match_template(image, template, 0)  # the context goes on beside it
+    torch.cuda.synchronize()
+    assert np.array_equal(bits(out.cpu().numpy()), bits(O.match_exact(image, template, 3, None, precision=0)))
