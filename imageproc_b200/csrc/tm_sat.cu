@@ -30,6 +30,7 @@
 // rescan with offsets).
 #include "tm_common.cuh"
 #include "tm_internal.h"
+#include "tm_strip.h"
 
 namespace ipb {
 namespace {
@@ -150,7 +151,7 @@ __global__ void __launch_bounds__(32 * kSegs) sat_cols_kernel(uint32_t cols, uin
   }
 }
 
-constexpr uint32_t kStripRows = 16, kTileCols = 1024, kTileThreads = 256;
+constexpr uint32_t kTileCols = 1024, kTileThreads = 256;
 
 // A thread's four pixels at x of each of a strip's first n rows, zero past the
 // image: one word per row where rows are word-aligned, else the two aligned
@@ -166,7 +167,7 @@ __device__ __forceinline__ void strip_pixels(const uint8_t* __restrict__ img, ui
 #pragma unroll
     for (uint32_t r = 0; r < kStripRows; ++r)
       v[r] = r < n && in ? __ldg(reinterpret_cast<const uint32_t*>(p + (size_t)r * W)) : 0u;
-  } else if (y0 && y0 + kStripRows < H) {
+  } else if (strip_words_inside(W, H, y0)) {
 #pragma unroll
     for (uint32_t r = 0; r < kStripRows; ++r) {
       const uint8_t* g = p + (size_t)r * W;

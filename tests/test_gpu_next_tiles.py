@@ -86,6 +86,30 @@ def test_integral_unaligned_device_buffers_and_capture():
         assert np.array_equal(out.cpu().numpy(), exp)
 
 
+@pytest.mark.parametrize("W,H", [(1, 2001), (2, 2002), (3, 2017), (5, 2017), (1028, 1290), (1030, 2409), (2049, 2801)])
+def test_integral_strips_unaligned_device_buffers_and_capture(W, H):
+    # tall enough for the strips at every base address: the last words of narrow
+    # images, a poisoned table, and the call inside a graph
+    import torch
+    fn = _lib.lib().ipb_integral_image_device
+    fn.argtypes = [C.c_void_p, C.c_uint32, C.c_uint32, C.c_uint32, C.c_int, C.c_int, C.c_void_p, C.c_void_p]
+    fn.restype = C.c_int
+    img = np.random.default_rng(W).integers(0, 256, (H, W), dtype=np.uint8)
+    exp = np.zeros((H + 1, W + 1), np.int64)
+    exp[1:, 1:] = (img.astype(np.int64) ** 2).cumsum(0).cumsum(1)
+    for off in range(4):
+        buf = torch.full((H * W + 8,), 255, dtype=torch.uint8, device="cuda")
+        d = buf[off:off + H * W]
+        d.copy_(torch.from_numpy(img.reshape(-1)))
+        out = torch.full((H + 1, W + 1), -1, dtype=torch.int64, device="cuda")
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            _lib.check(fn(d.data_ptr(), W, H, 1, 1, 64, out.data_ptr(), torch.cuda.current_stream().cuda_stream))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(out.cpu().numpy(), exp), off
+
+
 @pytest.mark.parametrize("dtype", [np.uint8, np.int8, np.uint16, np.int16, np.uint32, np.int32, np.float32])
 def test_suppress_every_radius_and_lowest_values(dtype):
     g = np.random.default_rng(np.dtype(dtype).num)

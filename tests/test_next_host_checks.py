@@ -5,6 +5,8 @@ with the reference's panic messages where the reference panics, and the empty
 inputs that need no device at all.
 """
 
+from pathlib import Path
+
 import numpy as np
 import pytest
 
@@ -76,3 +78,16 @@ def test_integral_images_reject_unsupported_arrays():
         II.integral_image(np.zeros((4, 5, 2), np.uint8))
     with pytest.raises(TypeError):
         II.integral_squared_image(IMG, dtype=np.uint16)
+
+
+def test_strip_words_stay_inside_narrow_images(tmp_path):
+    import shutil
+    import subprocess
+    if not shutil.which("g++"):
+        pytest.skip("no C++ compiler")
+    root = Path(__file__).resolve().parents[1]
+    exe = tmp_path / "strip_words"
+    subprocess.run(["g++", "-std=c++17", "-I", str(root / "imageproc_b200" / "csrc"),
+                    str(root / "tests" / "cpp" / "strip_words.cpp"), "-o", str(exe)], check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout + r.stderr
