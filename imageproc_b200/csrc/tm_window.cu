@@ -1252,12 +1252,16 @@ cudaError_t launch_window_batch(const WindowPlan& pl, WindowLaunch& L, cudaStrea
 }
 
 // Estimated cycles of one launch of n problems in tiles of 16 nj rows and sets
-// of up to `set`: waves of tiles x (a set's MMAs and its epilogues) + set-up.
-// An SS MMA of 128 x N x 32 takes max(32 + N/4, N/2); an epilogue about 1000
-// per 16 output rows. Against 1080p and 512 x 512 maps with templates of 8 to
-// 128 pixels a side the estimate puts the fastest height and set within 1.25
-// of its least (four 64 x 64 templates at 1080p, sets of 4: 128 rows 57 us, 64
-// rows 79; alone: 72 and 85; at 512 x 512, 16 x 16: 27, 20, 17 and 13).
+// of up to `set`: waves of tiles x (what a tile costs whatever its height, a
+// set's MMAs and its epilogues) + set-up. An SS MMA of 128 x N x 32 takes
+// max(32 + N/4, N/2); a tile about 2000, its epilogue about 600 per 16 output
+// rows. Those two were fitted to single maps timed at every height (59 images
+// of 91 x 107 to 4100 x 3000 with 21 templates of 1 to 128 a side, masked or
+// not): the height of the least estimate is 0.1 % slower than the fastest on
+// average, at most 1.23 times. Without the tile's own cost, small templates on
+// images of more tiles than SMs were cut into tiles of 16 rows (1280 x 957, 16
+// x 16, CrossCorrelationNormalized: 27 us, 128 rows 19, the Hankel-row kernel
+// 24).
 double window_cost(const MatchArgs* const* a, uint32_t n, uint32_t nj, uint32_t set) {
   const double sms = (double)device_sm_count(), mma = std::max(32.0 + 4.0 * nj, 8.0 * nj);
   double tiles = 0, work = 0;
@@ -1266,7 +1270,7 @@ double window_cost(const MatchArgs* const* a, uint32_t n, uint32_t nj, uint32_t 
     const double t = (double)(((q.W - q.w) / kTileW + 1) * (uint64_t)((q.H - q.h) / (16 * nj) + 1));
     const double corr = 1.0 + (q.mask && q.method != IPB_CROSS_CORRELATION ? 2.0 / set : 0.0);
     tiles += t / set;
-    work += t * (corr * (k_of(q.w) / 32) * (q.h + 7.0) * mma + 1000.0 * nj);
+    work += t * (2000.0 / set + corr * (k_of(q.w) / 32) * (q.h + 7.0) * mma + 600.0 * nj);
   }
   return work / tiles * std::ceil(tiles / sms) + 6000.0;
 }

@@ -173,3 +173,22 @@ def test_window_kernel_short_tiles(rows, members, tmp_path, monkeypatch):
         assert bad.size == 0, (k, bad[:3])
     plan.close()
     _lib.lib().ipb_batch_tuning_reset()
+
+
+@pytest.mark.parametrize("W,H,w,h,rows", [(1280, 957, 16, 16, 128), (1283, 957, 8, 8, 128), (512, 512, 16, 16, 16),
+                                          (4095, 3000, 9, 16, 128)])
+def test_estimate_counts_a_tiles_own_cost(W, H, w, h, rows, monkeypatch):
+    # measured, 16 to 128 rows per tile: 1280 x 957 27, 22, 20 and 19 us, 1283 x
+    # 957 26, 18, 18 and 16, 512 x 512 12, 13, 17 and 20, 4095 x 3000 180, 104,
+    # 73 and 60
+    import torch
+
+    from imageproc_b200 import _lib, device
+    monkeypatch.setenv("IPB_AUTOTUNE", "0")
+    monkeypatch.setenv("IPB_TUNING_FILE", "")
+    _lib.lib().ipb_batch_tuning_reset()
+    image, template, _ = scene(W, H, w, h)
+    batch = device.Batch([(torch.from_numpy(image).cuda(), torch.from_numpy(template).cuda(), 0)], extremes=False)
+    plan = device.BatchPlan(batch)
+    assert [g["tile_rows"] for g in plan.info()["launches"]] == [rows]
+    plan.close()
