@@ -10,7 +10,8 @@
 // contraction) and wrapping two's-complement arithmetic for i32 kernels (a
 // release build).
 //
-// Kernels up to 8 columns by 32 rows: filter_rows_kernel. A row of the image
+// Kernels up to 8 columns by 32 rows on images of more blocks than run at
+// once: filter_rows_kernel. A row of the image
 // is W * C elements, a tap k_x columns away is k_x * C elements away, so one
 // kernel serves every channel count. A block stages its clamped input window
 // once, converted to the kernel's type, in shared memory; a thread owns 4
@@ -20,11 +21,12 @@
 // operations per tap (no fused multiply-add): 4096 x 4096 u8, 5 x 5 f32 to u8,
 // 23 us at the FP32 issue rate. Against one thread per pixel reading a byte and
 // converting it per tap: 209 -> 56 us.
-// Larger kernels: filter_tile_kernel (to 64 x 64, a 32 x 8 output tile and its
-// input window as bytes) and filter_global_kernel.
+// Smaller images and larger kernels: filter_tile_kernel (to 64 x 64, a 32 x 8
+// output tile and its input window as bytes) and filter_global_kernel.
 #include <type_traits>
 
 #include "tm_common.cuh"
+#include "tm_filter_rule.h"
 #include "tm_internal.h"
 
 namespace ipb {
@@ -32,7 +34,7 @@ namespace {
 
 __device__ __forceinline__ uint32_t align_up_dev(uint32_t v, uint32_t a) { return (v + a - 1) / a * a; }
 
-constexpr int kTX = 32, kTY = 8;
+constexpr int kTX = kFilterTileW, kTY = kFilterTileH;
 constexpr uint32_t kMaxTileKernel = 64;  // kernels up to 64 x 64 use the shared-memory tile
 
 // Clamp<K> for S (src/definitions.rs:119-190): values at or above the maximum
@@ -128,16 +130,10 @@ __global__ void __launch_bounds__(kTX* kTY) filter_global_kernel(const uint8_t* 
   for (int c = 0; c < C; ++c) out[((size_t)y * W + x) * C + c] = clamp_to<S>(acc[c]);
 }
 
-constexpr int kRowVec = 4, kRowRows = 4;          // elements and rows per thread
-constexpr uint32_t kRowTile = 32 * kRowVec;      // elements per block row
-constexpr uint32_t kRowMaxW = 8, kRowMaxH = 32;  // taps
-
-// Elements staged ahead of the tile: the leftmost tap's, rounded up to a word.
-__host__ __device__ constexpr uint32_t row_pad(uint32_t C, uint32_t KW) { return ((KW / 2) * C + 3) & ~3u; }
-// Staged elements per row: the tile, the pad and the taps to the right.
-__host__ __device__ constexpr uint32_t row_pitch(uint32_t C, uint32_t KW) {
-  return row_pad(C, KW) + ((kRowTile + (KW - 1 - KW / 2) * C + 3) & ~3u);
-}
+constexpr int kRowVec = 4, kRowRows = kFilterStripRows;  // elements and rows per thread
+constexpr uint32_t kRowTile = kFilterStripW;              // elements per block row
+constexpr uint32_t kRowMaxW = 8, kRowMaxH = 32;           // taps
+static_assert(kRowTile == 32 * kRowVec, "a warp per strip row");
 
 template <typename K>
 __device__ __forceinline__ K from_byte(uint32_t word, int k) {
@@ -166,12 +162,13 @@ __device__ __forceinline__ void store_vec(void* out, size_t at, const K (&acc)[k
 }
 
 // in_aligned / out_aligned: every row starts on a 4-element boundary.
+// (kPitch * C is a multiple of C above any distance to the left of a row.)
 template <int C, int KW, typename K>
 __global__ void __launch_bounds__(256) filter_rows_kernel(const uint8_t* __restrict__ img, uint32_t W, uint32_t H,
                                                          const K* __restrict__ kern, uint32_t kh, int otype,
                                                          bool in_aligned, bool out_aligned, void* __restrict__ out) {
   extern __shared__ __align__(16) uint8_t smem[];
-  constexpr uint32_t kPad = row_pad(C, KW), kPitch = row_pitch(C, KW), kWords = kPitch / 4;
+  constexpr uint32_t kPad = filter_strip_pad(C, KW), kPitch = filter_strip_pitch(C, KW), kWords = kPitch / 4;
   constexpr uint32_t kFirst = kPad - (KW / 2) * C;           // the leftmost tap of element 0
   constexpr uint32_t kLast = kFirst + kRowVec + (KW - 1) * C;  // elements a thread reads per row
   constexpr uint32_t kVecs = (kLast + 3) / 4, kTaps = (KW + 3) & ~3;
@@ -200,9 +197,11 @@ __global__ void __launch_bounds__(256) filter_rows_kernel(const uint8_t* __restr
     } else {
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        long long x = e + k;  // the same channel of the nearest pixel
-        if (x < 0) x = (x % C + C) % C;
-        else if (x >= n) x = n - C + x % C;
+        // the same channel of the nearest pixel; past the ends by no more than
+        // a staged row, so the remainders are of 32 bits
+        long long x = e + k;
+        if (x < 0) x = (int)(x + (long long)(kPitch * C)) % C;
+        else if (x >= n) x = n - C + (int)(x - n) % C;
         v |= (uint32_t)__ldg(row + x) << (8 * k);
       }
     }
@@ -261,23 +260,12 @@ __global__ void __launch_bounds__(256) filter_rows_kernel(const uint8_t* __restr
 }
 
 template <int C, int KW, typename K>
-cudaError_t launch_filter_rows_k(const uint8_t* img, uint32_t W, uint32_t H, const K* kern, uint32_t kh, int otype,
-                                 size_t osize, void* out, cudaStream_t s) {
+cudaError_t launch_filter_rows_k(const uint8_t* img, uint32_t W, uint32_t H, const K* kern, uint32_t kh, uint32_t by,
+                                 int otype, size_t osize, void* out, cudaStream_t s) {
   const uint64_t n = (uint64_t)W * C;
-  const uint32_t gx = (uint32_t)((n + kRowTile - 1) / kRowTile);
-  // 32 rows per block (the halo rows are a small share), 8 where the image
-  // would give an SM less than two blocks
-  uint32_t by = 8;
-  if ((uint64_t)gx * ((H + 31) / 32) < 2ull * (uint32_t)device_sm_count()) by = 2;
-  while (by < 8 && (H + by * kRowRows - 1) / (by * kRowRows) > 65535u) by *= 2;
-  const uint32_t rows = by * kRowRows, gy = (H + rows - 1) / rows;
-  if (gy > 65535u) return cudaErrorInvalidValue;
-  const size_t smem = sizeof(K) * ((size_t)kh * ((KW + 3) & ~3) + (size_t)(rows + kh - 1) * row_pitch(C, KW));
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(filter_rows_kernel<C, KW, K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e != cudaSuccess) return e;
-  }
+  const uint32_t rows = by * kRowRows, gx = (uint32_t)((n + kRowTile - 1) / kRowTile), gy = (H + rows - 1) / rows;
+  // at most 40 KB: 4 channels, 8 x 32 taps, 32 rows
+  const size_t smem = sizeof(K) * ((size_t)kh * ((KW + 3) & ~3) + (size_t)(rows + kh - 1) * filter_strip_pitch(C, KW));
   const bool in_aligned = n % 4 == 0 && (reinterpret_cast<uintptr_t>(img) & 3u) == 0;
   const bool out_aligned = n % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & (4 * osize - 1)) == 0;
   filter_rows_kernel<C, KW, K><<<dim3(gx, gy), dim3(32, by), smem, s>>>(img, W, H, kern, kh, otype, in_aligned,
@@ -288,17 +276,17 @@ cudaError_t launch_filter_rows_k(const uint8_t* img, uint32_t W, uint32_t H, con
 
 template <int C, typename K>
 cudaError_t launch_filter_rows(const uint8_t* img, uint32_t W, uint32_t H, const void* kern, uint32_t kw, uint32_t kh,
-                               int otype, size_t osize, void* out, cudaStream_t s) {
+                               uint32_t by, int otype, size_t osize, void* out, cudaStream_t s) {
   const K* k = static_cast<const K*>(kern);
   switch (kw) {
-    case 1: return launch_filter_rows_k<C, 1, K>(img, W, H, k, kh, otype, osize, out, s);
-    case 2: return launch_filter_rows_k<C, 2, K>(img, W, H, k, kh, otype, osize, out, s);
-    case 3: return launch_filter_rows_k<C, 3, K>(img, W, H, k, kh, otype, osize, out, s);
-    case 4: return launch_filter_rows_k<C, 4, K>(img, W, H, k, kh, otype, osize, out, s);
-    case 5: return launch_filter_rows_k<C, 5, K>(img, W, H, k, kh, otype, osize, out, s);
-    case 6: return launch_filter_rows_k<C, 6, K>(img, W, H, k, kh, otype, osize, out, s);
-    case 7: return launch_filter_rows_k<C, 7, K>(img, W, H, k, kh, otype, osize, out, s);
-    default: return launch_filter_rows_k<C, 8, K>(img, W, H, k, kh, otype, osize, out, s);
+    case 1: return launch_filter_rows_k<C, 1, K>(img, W, H, k, kh, by, otype, osize, out, s);
+    case 2: return launch_filter_rows_k<C, 2, K>(img, W, H, k, kh, by, otype, osize, out, s);
+    case 3: return launch_filter_rows_k<C, 3, K>(img, W, H, k, kh, by, otype, osize, out, s);
+    case 4: return launch_filter_rows_k<C, 4, K>(img, W, H, k, kh, by, otype, osize, out, s);
+    case 5: return launch_filter_rows_k<C, 5, K>(img, W, H, k, kh, by, otype, osize, out, s);
+    case 6: return launch_filter_rows_k<C, 6, K>(img, W, H, k, kh, by, otype, osize, out, s);
+    case 7: return launch_filter_rows_k<C, 7, K>(img, W, H, k, kh, by, otype, osize, out, s);
+    default: return launch_filter_rows_k<C, 8, K>(img, W, H, k, kh, by, otype, osize, out, s);
   }
 }
 
@@ -308,7 +296,8 @@ cudaError_t launch_filter_t(const uint8_t* img, uint32_t W, uint32_t H, const vo
   const dim3 grid((W + kTX - 1) / kTX, (H + kTY - 1) / kTY), block(kTX, kTY);
   if (grid.y > 65535u) return cudaErrorInvalidValue;
   if (kw <= kRowMaxW && kh <= kRowMaxH)
-    return launch_filter_rows<C, K>(img, W, H, kern, kw, kh, elem_of<S>(), sizeof(S), out, s);
+    if (const uint32_t by = filter_strip_warps(W, H, C, kw, kh, (uint32_t)device_sm_count()))
+      return launch_filter_rows<C, K>(img, W, H, kern, kw, kh, by, elem_of<S>(), sizeof(S), out, s);
   const K* k = static_cast<const K*>(kern);
   S* o = static_cast<S*>(out);
   if (kw <= kMaxTileKernel && kh <= kMaxTileKernel) {

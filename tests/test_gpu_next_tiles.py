@@ -32,6 +32,22 @@ def test_filter_strips(channels, kw, kh):
             assert np.array_equal(got.view(np.uint8), exp.view(np.uint8)), (W, H, od)
 
 
+@pytest.mark.parametrize("channels", [1, 3, 4])
+@pytest.mark.parametrize("kw,kh", [(1, 1), (2, 3), (3, 32), (5, 5), (7, 1), (8, 7), (8, 32)])
+def test_filter_strips_of_large_images(channels, kw, kh):
+    # images that take the strips, in blocks of 8 and of 32 rows: rows on and off
+    # word boundaries, one element or row past a block, strips that both ends of
+    # a row clamp
+    g = np.random.default_rng(kw * 100 + kh)
+    for W, H in ((1027, 801), (1152, 797), (129, 8001), (6000, 41), (42, 16003)):
+        img = g.integers(0, 256, (H, W) if channels == 1 else (H, W, channels), dtype=np.uint8)
+        kf = g.standard_normal((kh, kw)).astype(np.float32)
+        ki = g.integers(-2**20, 2**20, (kh, kw)).astype(np.int32)
+        for k, od in ((kf, np.uint8), (kf, np.float32), (ki, np.int16), (ki, np.int32)):
+            got, exp = fl.filter_clamped(img, k, od), O.filter_clamped(img, k, od)
+            assert np.array_equal(got.view(np.uint8), exp.view(np.uint8)), (W, H, od)
+
+
 def test_filter_large_grid_rows():
     g = np.random.default_rng(3)
     img = g.integers(0, 256, (2051, 2053), dtype=np.uint8)  # 32-row blocks

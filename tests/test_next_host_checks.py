@@ -80,14 +80,22 @@ def test_integral_images_reject_unsupported_arrays():
         II.integral_squared_image(IMG, dtype=np.uint16)
 
 
-def test_strip_words_stay_inside_narrow_images(tmp_path):
+def _run_cpp(name, tmp_path):
     import shutil
     import subprocess
     if not shutil.which("g++"):
         pytest.skip("no C++ compiler")
     root = Path(__file__).resolve().parents[1]
-    exe = tmp_path / "strip_words"
+    exe = tmp_path / name
     subprocess.run(["g++", "-std=c++17", "-I", str(root / "imageproc_b200" / "csrc"),
-                    str(root / "tests" / "cpp" / "strip_words.cpp"), "-o", str(exe)], check=True)
+                    str(root / "tests" / "cpp" / f"{name}.cpp"), "-o", str(exe)], check=True)
     r = subprocess.run([str(exe)], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_strip_words_stay_inside_narrow_images(tmp_path):
+    _run_cpp("strip_words", tmp_path)
+
+
+def test_filter_kernel_choice(tmp_path):
+    _run_cpp("filter_rule", tmp_path)
