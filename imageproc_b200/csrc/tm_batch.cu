@@ -270,11 +270,10 @@ ipb_status to_status(cudaError_t e, const char* what) {
     if (e_ != cudaSuccess) return to_status(e_, what); \
   } while (0)
 
-// Descriptors of a window-kernel group in tiles of `rows` output rows; false
-// when no plan fits.
-template <class KeysOf>
-bool window_group(const ipb_batch_plan* p, const std::vector<uint32_t>& mem, bool masked, uint32_t rows, uint32_t set,
-                  KeysOf keys_of, ipb_batch_plan::Group& g) {
+// Plan of a window-kernel group in tiles of `rows` output rows; false when none
+// fits.
+bool window_plan_rows(const ipb_batch_plan* p, const std::vector<uint32_t>& mem, bool masked, uint32_t rows,
+                      WindowPlan& pl) {
   uint32_t wmax = 1, hmax = 1;
   for (uint32_t i : mem) {
     if (!window_supported(p->args[i])) return false;
@@ -282,7 +281,14 @@ bool window_group(const ipb_batch_plan* p, const std::vector<uint32_t>& mem, boo
     hmax = std::max(hmax, p->args[i].h);
   }
   if (rows != 16 && rows != 32 && rows != 64 && rows != 128) return false;
-  if (!window_plan_best(wmax, hmax, masked, rows / 16, g.wplan)) return false;
+  return window_plan_best(wmax, hmax, masked, rows / 16, pl);
+}
+
+// Its descriptors.
+template <class KeysOf>
+bool window_group(const ipb_batch_plan* p, const std::vector<uint32_t>& mem, bool masked, uint32_t rows, uint32_t set,
+                  KeysOf keys_of, ipb_batch_plan::Group& g) {
+  if (!window_plan_rows(p, mem, masked, rows, g.wplan)) return false;
   g.window = true;
   g.set = set;
   g.wprobs.clear();
@@ -763,6 +769,10 @@ ipb_status create(const ipb_pair* pairs, uint32_t n, int precision, bool capture
           have = true;
         }
       }
+      // a height cached for narrower templates of the same key may leave no room
+      // for this group's: the estimate's choice then, and the cache stays
+      WindowPlan fits;
+      if (have && window && c.ks == 0 && !window_plan_rows(p, mem, masked, c.nt, fits)) c = choices.front();
       if (!have) {
         ipb_status st = window ? tune_window_group(p, mem, masked, choices, keys_of, c)
                                : tune_group(p, mem, ks0, masked, hmax, set, keys_of, c);

@@ -192,3 +192,38 @@ def test_estimate_counts_a_tiles_own_cost(W, H, w, h, rows, monkeypatch):
     plan = device.BatchPlan(batch)
     assert [g["tile_rows"] for g in plan.info()["launches"]] == [rows]
     plan.close()
+
+
+def test_cached_height_without_a_plan_falls_back_to_the_estimate(tmp_path, monkeypatch):
+    # 128 rows fit masked templates of up to 113 x 64, and a narrower one of the
+    # same key may have left them in the file: a 128 x 64 one takes what it would
+    # take without a file
+    import torch
+
+    from imageproc_b200 import _lib, device
+    W, H, w, h = 1920, 1080, 128, 64  # more tiles than SMs: the estimate makes sets of two
+    image, t0, mask = scene(W, H, w, h)
+    di, d0, dm = (torch.from_numpy(a).cuda() for a in (image, t0, mask))
+    batch = device.Batch([(di, d0, k, dm) for k in (1, 3)])
+    monkeypatch.setenv("IPB_AUTOTUNE", "0")
+    monkeypatch.setenv("IPB_TUNING_FILE", "")
+    _lib.lib().ipb_batch_tuning_reset()
+    plan = device.BatchPlan(batch)
+    untuned = plan.info()["launches"]
+    plan.close()
+    pos = 2 * (W - w + 1) * (H - h + 1)
+    f = tmp_path / "tuning.txt"
+    line = f"group2 32 1 {h} {pos.bit_length() - 1} 10 102 0 128 1\n"
+    f.write_text(line)
+    monkeypatch.setenv("IPB_TUNING_FILE", str(f))
+    monkeypatch.delenv("IPB_AUTOTUNE")
+    _lib.lib().ipb_batch_tuning_reset()
+    plan = device.BatchPlan(batch)
+    assert f.read_text() == line  # the key was found
+    assert plan.info()["launches"] == untuned and untuned[0]["set_size"] == 2
+    plan.launch()
+    torch.cuda.synchronize()
+    for k, out in zip((1, 3), batch.outs):
+        assert np.array_equal(bits(out.cpu().numpy()), bits(O.match_exact(image, t0, k, mask, precision=0)))
+    plan.close()
+    _lib.lib().ipb_batch_tuning_reset()
