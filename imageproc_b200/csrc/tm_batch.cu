@@ -108,8 +108,10 @@ namespace {
 //    its largest image side, largest set, plus 100 for the window kernel).
 //    Line: "group2 ks0 masked h8 wlog mlog set ks nt n".
 //  * per pair shape class (IPB_AUTOTUNE=1): tensor cores or the CUDA-core
-//    kernel, timed on the first pair of each (w, h, masked, normalised).
-//    Line: "pair w h masked norm tensor".
+//    kernel, timed on the first pair of each (w, h, masked, normalised) with
+//    the kernel that the pair would run on.
+//    Line: "pair2 w h masked norm tensor" (a "pair" line is of the time when
+//    the Hankel-row kernel took every pair, and is not read).
 struct TuneKey {
   uint32_t w, h;
   int masked, norm;
@@ -155,7 +157,7 @@ void tune_load_locked() {
     std::istringstream ls(line);
     std::string kind;
     ls >> kind;
-    if (kind == "pair") {
+    if (kind == "pair2") {
       TuneKey k;
       int t;
       if (ls >> k.w >> k.h >> k.masked >> k.norm >> t) g_tune[k] = t != 0;
@@ -176,7 +178,7 @@ void tune_store_locked() {
   {
     std::ofstream out(tmp);
     for (auto& kv : g_tune)
-      out << "pair " << kv.first.w << ' ' << kv.first.h << ' ' << kv.first.masked << ' ' << kv.first.norm << ' '
+      out << "pair2 " << kv.first.w << ' ' << kv.first.h << ' ' << kv.first.masked << ' ' << kv.first.norm << ' '
           << (kv.second ? 1 : 0) << '\n';
     for (auto& kv : g_group_tune)
       out << "group2 " << kv.first.ks0 << ' ' << kv.first.masked << ' ' << kv.first.h8 << ' ' << kv.first.wlog
@@ -212,8 +214,10 @@ uint32_t floor_log2(double v) {
   return l;
 }
 
-// Cost model: tensor cores whenever the shape is supported (they win from
-// 16x8 templates up; below that the CUDA-core kernel takes the pair).
+// Cost model: tensor cores whenever the Hankel-row kernel supports the shape (8
+// pixels a side and more). Smaller templates run on the CUDA-core kernel here.
+// In single calls the window kernel takes them, and it is the faster one (7 x 7
+// at 1080p: 15 against 113 us); groups of them are not formed.
 bool model_prefers_tensor(const MatchArgs& a) { return umma_supported(a); }
 
 float time_launch(const MatchArgs& a, bool tensor, void* scratch, unsigned int* err) {
@@ -223,8 +227,9 @@ float time_launch(const MatchArgs& a, bool tensor, void* scratch, unsigned int* 
   float best = 1e30f;
   for (int rep = 0; rep < 3; ++rep) {
     cudaEventRecord(e0, a.stream);
-    if (tensor) launch_umma(a, err, 0);
-    else launch_exact_cc(a, scratch);
+    if (!tensor) launch_exact_cc(a, scratch);
+    else if (kernel_path() == 0 && window_supported(a)) launch_window(a, err, 0);
+    else launch_umma(a, err, 0);
     cudaEventRecord(e1, a.stream);
     cudaEventSynchronize(e1);
     float ms = 0;

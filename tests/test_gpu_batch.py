@@ -230,6 +230,31 @@ def test_batch_tuner_persists_choices_and_replays_rearm_extremes(tmp_path, monke
     L.ipb_batch_tuning_reset()
 
 
+def test_pair_choice_is_of_the_kernel_that_runs(tmp_path, monkeypatch):
+    # a decision persisted when the Hankel-row kernel was timed does not apply to
+    # pairs that the window kernel takes
+    import torch
+
+    from imageproc_b200 import device
+    L = _lib.lib()
+    f = tmp_path / "tuning.txt"
+    f.write_text("pair 64 64 0 0 0\n")  # "the CUDA cores are faster"
+    monkeypatch.setenv("IPB_TUNING_FILE", str(f))
+    monkeypatch.setenv("IPB_AUTOTUNE", "1")
+    L.ipb_batch_tuning_reset()
+    g = np.random.default_rng(64)
+    items = [(g.integers(0, 256, (700, 900), dtype=np.uint8), g.integers(0, 256, (64, 64), dtype=np.uint8), 0, None)]
+    batch = device.Batch(_to_device(items))
+    plan = device.BatchPlan(batch)
+    assert plan.info()["tensor_pairs"] == 1
+    assert "pair2 64 64 0 0 1\n" in f.read_text()
+    plan.launch()
+    torch.cuda.synchronize()
+    _check(items, batch.outs, batch.extremes_host())
+    plan.close()
+    L.ipb_batch_tuning_reset()
+
+
 def _shared_image_items(seed):
     """Pairs that share images: per image, classes of 1..8 pairs with one
     template size (own template content, methods, binary masks or none), a
