@@ -123,3 +123,28 @@ def test_set_plans_of_the_headline_shapes():
     p = _lib.tensor_set_plan(64, 64, True, 4)
     assert (p["tile_rows"], p["rows_per_stage"], p["tmem_columns"]) == (64, 2, 5 * 64 + 2 * 3 * 16 * 2)
     assert _lib.tensor_set_plan(64, 64, False, 5) is None
+
+
+@pytest.mark.parametrize("rows", [16, 64, 128])
+@pytest.mark.parametrize("w,h", [(64, 64), (17, 5), (18, 128), (1, 1)])
+def test_bench_counts_the_macs_of_the_window_kernel(w, h, rows):
+    # per tile, step rho feeds D[m][n] += sum_k A_rho[m][k] B_rho[n][k] with 128
+    # lanes m, a column n per 8 x 16 block of outputs and K bytes of k
+    import importlib
+    import sys
+    from pathlib import Path
+    root = str(Path(__file__).resolve().parents[1])
+    if root not in sys.path:
+        sys.path.insert(0, root)
+    ratio = importlib.import_module("bench").executed_mac_ratio
+    W, H = 700, 300
+    Wo, Ho = W - w + 1, H - h + 1
+    macs = 0
+    for y0 in range(0, Ho, rows):
+        for x0 in range(0, Wo, 128):
+            for rho in range(h + 7):
+                macs += 128 * (128 // 16 * rows // 8) * next(k for k in range(32, 999, 32) if k >= w + 15)
+    for masked, set_size, corr in ((False, 4, 1.0), (True, 4, 1.5), (True, 1, 3.0)):
+        got = ratio(W, H, w, h, masked, rows, set_size)
+        assert got["ratio"] == pytest.approx(corr * macs / (Wo * Ho * w * h), rel=1e-12)
+        assert (got["tile_rows"], got["set_size"]) == (rows, set_size)
