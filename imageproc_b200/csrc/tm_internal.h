@@ -66,7 +66,7 @@ enum KernelId : int {
   kKernelTemplateSumF32,
   kKernelReference,
   kKernelExtremes,
-  kKernelUmma,
+  kKernelUmma,  // the tensor-core exact kernels: window and Hankel-row
   kKernelMany,
   kKernelSuppress,
   kKernelFilter,
@@ -292,7 +292,7 @@ cudaError_t launch_extremes_keys_init(unsigned long long* keys, uint32_t n, cuda
 cudaError_t launch_extremes_keys_finish(unsigned long long* keys, const uint32_t* widths,
                                         ipb_extremes_f32* const* outs, uint32_t n, cudaStream_t s);
 
-// ---- tensor-core exact kernel with the staged tile as the A operand (tm_window.cu)
+// ---- tensor-core exact kernel with the staged tile as the B operand (tm_window.cu)
 // One problem of a launch (device-side descriptor).
 struct WindowProblem {
   const uint8_t* img;

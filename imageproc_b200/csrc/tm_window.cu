@@ -1083,11 +1083,10 @@ uint32_t pitch_of(uint32_t w) { return (kTileW - 1 + w + 15) & ~15u; }
 
 }  // namespace
 
-// Every template of up to 128 x 128, the smallest included: against the
-// CUDA-core kernel, SumOfSquaredErrors with 1 x 1, 7 x 7 and 1 x 64 templates
-// takes 12, 12 and 12 us where that takes 50, 52 and 75 (512 x 512), and 52, 58
-// and 57 where it takes 472, 492 and 797 (4096 x 3000). Masked, the nearest is
-// 1 x 1 on 1283 x 957, 26 and 25 us.
+// Every template of up to 128 x 128, the smallest included: SumOfSquaredErrors
+// with 1 x 1, 7 x 7 and 1 x 64 templates takes 12, 12 and 12 us where the
+// CUDA-core kernel takes 50, 52 and 75 (512 x 512), and 46, 48 and 58 where
+// that takes 472, 492 and 797 (4096 x 3000).
 bool window_supported(const MatchArgs& a) {
   if (a.precision == IPB_PRECISION_REFERENCE_F32 || (a.mask && !a.mask_binary)) return false;
   if (a.w < 1 || a.h < 1 || a.w > kMaxSide || a.h > kMaxSide || a.w > a.W || a.h > a.H) return false;
